@@ -11,6 +11,7 @@
 #include "solve.h"
 #include "harmonics.cuh"
 #include "mindlin_gen.cuh"
+#include "image_moments.cuh"
 #include "../../include/elfmm3d_b200.h"
 
 using namespace efmm;
@@ -1342,6 +1343,35 @@ extern "C" int efmm_mindlin_image_kernel(int layer, double lam, double mu, const
     mindlin_image_sl_blk(lam, mu, x[0], x[1], x[2], s[0], s[1], s[2], out);
   else if (layer == 1)
     mindlin_image_dl_blk(lam, mu, x[0], x[1], x[2], s[0], s[1], s[2], nrm[0], nrm[1], nrm[2], out);
+  else
+    return IER_BADARG;
+  return IER_OK;
+}
+
+// Host evaluation of the moment form of the same kernels (image_moments.cuh,
+// the form the device near field integrates) for nnode weighted source nodes.
+extern "C" int efmm_mindlin_image_moments(int layer, int strain, double lam, double mu, const double* x, int nnode,
+                                          const double* s, const double* w, const double* nrm, double* out) {
+  using namespace efmm;
+  if (!x || !s || !w || !out || nnode < 1 || (layer == 1 && !nrm)) return IER_BADARG;
+  ImageConst c;
+  image_const(lam, mu, c);
+  for (int k = 0; k < 27; k++) out[k] = 0.0;
+  auto run = [&](auto m, auto&& assemble) {
+    m.clear();
+    for (int q = 0; q < nnode; q++) {
+      ImageNode g;
+      image_node(x, s + 3 * q, g);
+      m.add(g, w[q]);
+    }
+    assemble(m);
+  };
+  if (layer == 0)
+    run(ImageSL{}, [&](const ImageSL& m) { image_sl_assemble(m, c, x[2], strain != 0, out); });
+  else if (layer == 1 && strain)
+    run(ImageDL<true>{}, [&](const ImageDL<true>& m) { image_dl_assemble<true>(m, c, x[2], nrm, out); });
+  else if (layer == 1)
+    run(ImageDL<false>{}, [&](const ImageDL<false>& m) { image_dl_assemble<false>(m, c, x[2], nrm, out); });
   else
     return IER_BADARG;
   return IER_OK;

@@ -29,7 +29,7 @@ struct Quad12 {
   double b[12][3];
   double w[12];
 };
-__host__ __device__ inline void quad12(Quad12& q) {
+__host__ __device__ constexpr void quad12(Quad12& q) {
   const double a1 = 0.2492867451709104212916386, w1 = 0.1167862757263793660252896;
   const double a2 = 0.0630890144915022283403316, w2 = 0.05084490637020681692093681;
   const double b3 = 0.05314504984481694735324967, c3 = 0.3103524510337844054166077,

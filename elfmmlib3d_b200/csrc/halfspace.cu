@@ -23,8 +23,11 @@
 // This direct sum (O(N M) pair integrals) is the check of the image FMM
 // (image.cu); the FMM's near field uses the same refined quadrature
 // (k_hs_store).
+#include <type_traits>
+
 #include "common.cuh"
 #include "mindlin_gen.cuh"
+#include "image_moments.cuh"
 #include "halfspace.h"
 
 namespace efmm {
@@ -43,6 +46,39 @@ constexpr int HS_ASTACK = 3 * HS_ADAPT_DEPTH + 1;
 double hs_quad_eps(int iprec) {
   const double e = iprec_eps(iprec);
   return e > 0.0 ? fmin(1e-6, 0.1 * e) : 1e-16;
+}
+
+// The sub-triangle of v0 along a path of halvings (2 bits each, the first in
+// the highest bits).
+__device__ __forceinline__ void hs_descend(const double* v0, unsigned int cd, int depth, double a[3], double b[3],
+                                           double c[3]) {
+  for (int d = 0; d < 3; d++) {
+    a[d] = v0[d];
+    b[d] = v0[3 + d];
+    c[d] = v0[6 + d];
+  }
+  for (int l = depth - 1; l >= 0; l--) {
+    const int k = (cd >> (2 * l)) & 3;
+    double ab[3], bc[3], ca[3];
+    for (int d = 0; d < 3; d++) {
+      ab[d] = 0.5 * (a[d] + b[d]);
+      bc[d] = 0.5 * (b[d] + c[d]);
+      ca[d] = 0.5 * (c[d] + a[d]);
+    }
+    for (int d = 0; d < 3; d++) {
+      if (k == 0) { b[d] = ab[d]; c[d] = ca[d]; }
+      else if (k == 1) { a[d] = ab[d]; c[d] = bc[d]; }
+      else if (k == 2) { a[d] = ca[d]; b[d] = bc[d]; }
+      else { a[d] = ab[d]; b[d] = bc[d]; c[d] = ca[d]; }
+    }
+  }
+}
+
+__device__ __forceinline__ double hs_area(const double* a, const double* b, const double* c) {
+  const double u[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
+  const double v[3] = {c[0] - a[0], c[1] - a[1], c[2] - a[2]};
+  const double cr[3] = {u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]};
+  return 0.5 * sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
 }
 
 // Adaptive integration of NOUT outputs (NG groups of NOUT / NG, each with its
@@ -71,29 +107,8 @@ __device__ __noinline__ void hs_adapt(const double* v0, double eps, const Quad12
     --top;
     const unsigned int cd = code[top];
     const int depth = dep[top];
-    // the sub-triangle: descend from v0 along the path (2 bits per halving,
-    // the first halving in the highest bits)
     double a[3], b[3], c[3];
-    for (int d = 0; d < 3; d++) {
-      a[d] = v0[d];
-      b[d] = v0[3 + d];
-      c[d] = v0[6 + d];
-    }
-    for (int l = depth - 1; l >= 0; l--) {
-      const int k = (cd >> (2 * l)) & 3;
-      double ab[3], bc[3], ca[3];
-      for (int d = 0; d < 3; d++) {
-        ab[d] = 0.5 * (a[d] + b[d]);
-        bc[d] = 0.5 * (b[d] + c[d]);
-        ca[d] = 0.5 * (c[d] + a[d]);
-      }
-      for (int d = 0; d < 3; d++) {
-        if (k == 0) { b[d] = ab[d]; c[d] = ca[d]; }
-        else if (k == 1) { a[d] = ab[d]; c[d] = bc[d]; }
-        else if (k == 2) { a[d] = ca[d]; b[d] = bc[d]; }
-        else { a[d] = ab[d]; b[d] = bc[d]; c[d] = ca[d]; }
-      }
-    }
+    hs_descend(v0, cd, depth, a, b, c);
     double ab[3], bc[3], ca[3];
     for (int d = 0; d < 3; d++) {
       ab[d] = 0.5 * (a[d] + b[d]);
@@ -265,73 +280,65 @@ k_hs_image(int n, const HsTri* __restrict__ tris, int m, const double* __restric
   for (int d = 0; d < 6; d++) atomicAdd(e6 + 6 * (size_t)i + d, acc[3 + d]);
 }
 
-// Unit-density blocks of one (target, triangle) pair with the refinement of
-// hs_pair: acc[0..26] single layer (unit force e_k at 9k), acc[27..53]
-// double layer (unit jump e_p at 27 + 9p); displacement then strain.
-__device__ void hs_pair_blk(const double* tv, const double nrm[3], const double X[3], int dosl, int dodl,
-                            double lam, double mu, const Quad12& Q, double eps, int* ncap, double* acc) {
+// ---------------------------------------------------- stored near field blocks
+namespace {
+constexpr Quad12 make_quad12() {
+  Quad12 q{};
+  quad12(q);
+  return q;
+}
+__constant__ Quad12 c_quad12 = make_quad12();
+}  // namespace
+
+// Moments of the 12-node rule on one sub-triangle, ADDED to m.
+template <class M>
+__device__ __forceinline__ void hs_rule(const double* a, const double* b, const double* c, const double X[3], M& m) {
+  const double area = hs_area(a, b, c);
+#pragma unroll 1
+  for (int q = 0; q < 12; q++) {
+    double y[3];
+    for (int d = 0; d < 3; d++)
+      y[d] = c_quad12.b[q][0] * a[d] + c_quad12.b[q][1] * b[d] + c_quad12.b[q][2] * c[d];
+    ImageNode g;
+    image_node(X, y, g);
+    m.add(g, c_quad12.w[q] * area);
+  }
+}
+
+// Moments m (ImageSL / ImageDL) of one (target, triangle) pair with the
+// refinement of hs_pair.  Near-singular sub-triangles are integrated
+// adaptively with error control on the responses, adapt(sub-triangle)
+// adding them to the pair's.
+template <class M, class Adapt>
+__device__ __forceinline__ void hs_pair_moments(const double* tv, const double X[3], M& m, Adapt adapt) {
   const double Xr[3] = {X[0], X[1], -X[2]};
   HsSub stk[HS_STACK];
   for (int c = 0; c < 9; c++) stk[0].v[c] = tv[c];
   stk[0].depth = 0;
   int top = 1;
+#pragma unroll 1
   while (top > 0) {
     const HsSub s = stk[--top];
     const double* a = s.v;
     const double* b = s.v + 3;
     const double* c = s.v + 6;
-    double cen[3], diam;
-    for (int d = 0; d < 3; d++) cen[d] = (a[d] + b[d] + c[d]) / 3.0;
+    double diam2, dist2 = 0;
     {
       double e0 = 0, e1 = 0, e2 = 0;
       for (int d = 0; d < 3; d++) {
+        const double cen = (a[d] + b[d] + c[d]) / 3.0;
+        dist2 += (Xr[d] - cen) * (Xr[d] - cen);
         e0 += (b[d] - a[d]) * (b[d] - a[d]);
         e1 += (c[d] - b[d]) * (c[d] - b[d]);
         e2 += (a[d] - c[d]) * (a[d] - c[d]);
       }
-      diam = sqrt(fmax(e0, fmax(e1, e2)));
+      diam2 = fmax(e0, fmax(e1, e2));
     }
-    double dist2 = 0;
-    for (int d = 0; d < 3; d++) dist2 += (Xr[d] - cen[d]) * (Xr[d] - cen[d]);
-    const bool far = dist2 > HS_RATIO * HS_RATIO * diam * diam;
+    const bool far = dist2 > HS_RATIO * HS_RATIO * diam2;
     if (!far && (s.depth >= HS_MAXDEPTH || top + 4 > HS_STACK)) {
-      // near-singular: each layer adaptively with error control per unit direction
-      if (dosl)
-        hs_adapt<27, 3>(s.v, eps, Q,
-                        [&](const double* y, double w, double* out) {
-                          double o[27];
-                          mindlin_image_sl_blk(lam, mu, X[0], X[1], X[2], y[0], y[1], y[2], o);
-                          for (int k = 0; k < 27; k++) out[k] += w * o[k];
-                        },
-                        acc, ncap);
-      if (dodl)
-        hs_adapt<27, 3>(s.v, eps, Q,
-                        [&](const double* y, double w, double* out) {
-                          double o[27];
-                          mindlin_image_dl_blk(lam, mu, X[0], X[1], X[2], y[0], y[1], y[2], nrm[0], nrm[1], nrm[2],
-                                               o);
-                          for (int k = 0; k < 27; k++) out[k] += w * o[k];
-                        },
-                        acc + 27, ncap);
+      adapt(s.v);
     } else if (far) {
-      const double u[3] = {b[0] - a[0], b[1] - a[1], b[2] - a[2]};
-      const double v[3] = {c[0] - a[0], c[1] - a[1], c[2] - a[2]};
-      const double cr[3] = {u[1] * v[2] - u[2] * v[1], u[2] * v[0] - u[0] * v[2], u[0] * v[1] - u[1] * v[0]};
-      const double area = 0.5 * sqrt(cr[0] * cr[0] + cr[1] * cr[1] + cr[2] * cr[2]);
-      for (int q = 0; q < 12; q++) {
-        double y[3];
-        for (int d = 0; d < 3; d++) y[d] = Q.b[q][0] * a[d] + Q.b[q][1] * b[d] + Q.b[q][2] * c[d];
-        const double w = Q.w[q] * area;
-        double o[27];
-        if (dosl) {
-          mindlin_image_sl_blk(lam, mu, X[0], X[1], X[2], y[0], y[1], y[2], o);
-          for (int k = 0; k < 27; k++) acc[k] += w * o[k];
-        }
-        if (dodl) {
-          mindlin_image_dl_blk(lam, mu, X[0], X[1], X[2], y[0], y[1], y[2], nrm[0], nrm[1], nrm[2], o);
-          for (int k = 0; k < 27; k++) acc[27 + k] += w * o[k];
-        }
-      }
+      hs_rule(a, b, c, X, m);
     } else {
       double ab[3], bc[3], ca[3];
       for (int d = 0; d < 3; d++) {
@@ -340,6 +347,7 @@ __device__ void hs_pair_blk(const double* tv, const double nrm[3], const double 
         ca[d] = 0.5 * (c[d] + a[d]);
       }
       const double* kids[4][3] = {{a, ab, ca}, {ab, b, bc}, {ca, bc, c}, {ab, bc, ca}};
+#pragma unroll
       for (int k = 0; k < 4; k++) {
         HsSub t;
         for (int vtx = 0; vtx < 3; vtx++)
@@ -351,9 +359,83 @@ __device__ void hs_pair_blk(const double* tv, const double nrm[3], const double 
   }
 }
 
-constexpr int HSS_PTS = 8;  // targets per CTA (the batched near-field chunks)
+// A near-singular sub-triangle v0: the unit responses of one layer (0
+// single, 1 double) with the adaptive scheme and error control of hs_adapt
+// (displacement and strain of each direction), ADDED to acc[27].
+template <int LAYER>
+__device__ __noinline__ void hs_adapt_blk(const double* v0, const double* nrm, const double X[3],
+                                          const ImageConst& cst, double eps, int* ncap, double* acc) {
+  using M = std::conditional_t<LAYER == 0, ImageSL, ImageDL<true>>;
+  auto assemble = [&](const M& m, double* o) {
+#pragma unroll
+    for (int k = 0; k < 27; k++) o[k] = 0.0;
+    if constexpr (LAYER == 0)
+      image_sl_assemble(m, cst, X[2], true, o);
+    else
+      image_dl_assemble<true>(m, cst, X[2], nrm, o);
+  };
+  unsigned int code[HS_ASTACK];
+  unsigned char dep[HS_ASTACK];
+  int top = 1;
+  code[0] = 0;
+  dep[0] = 0;
+#pragma unroll 1
+  while (top > 0) {
+    --top;
+    const unsigned int cd = code[top];
+    const int depth = dep[top];
+    double I[27], S[27];
+    // pass 0 the rule on the sub-triangle, pass 1 on its four children
+#pragma unroll 1
+    for (int pass = 0; pass < 2; pass++) {
+      M m;
+      m.clear();
+#pragma unroll 1
+      for (int k = 0; k < (pass ? 4 : 1); k++) {
+        double a[3], b[3], c[3];
+        hs_descend(v0, pass ? (cd << 2) | (unsigned int)k : cd, depth + pass, a, b, c);
+        hs_rule(a, b, c, X, m);
+      }
+      assemble(m, S);
+      if (pass == 0)
+        for (int k = 0; k < 27; k++) I[k] = S[k];
+    }
+    bool ok = true;
+    for (int g = 0; g < 3; g++) {
+      double dmax = 0.0, dif = 0.0;
+      for (int k = 9 * g; k < 9 * g + 9; k++) {
+        dmax = fmax(dmax, fabs(I[k]));
+        dif = fmax(dif, fabs(S[k] - I[k]));
+      }
+      ok = ok && dif <= eps * dmax;
+    }
+    if (ok || depth >= HS_ADAPT_DEPTH || top + 4 > HS_ASTACK) {
+      for (int k = 0; k < 27; k++) acc[k] += S[k];
+      if (!ok && ncap) atomicAdd(ncap, 1);
+      continue;
+    }
+    for (int k = 3; k >= 0; k--) {
+      code[top] = (cd << 2) | (unsigned int)k;
+      dep[top] = (unsigned char)(depth + 1);
+      top++;
+    }
+  }
+}
 
-__global__ void __launch_bounds__(128, 1)
+constexpr int HSS_PTS = 8;      // targets per chunk (the batched near-field chunks)
+constexpr int HSS_SLABS = 16;   // CTAs per chunk
+
+// Image near field blocks, one (target, near triangle) pair per thread; the
+// pairs of a chunk (8 targets of a leaf x its near triangles) are dealt to
+// HSS_SLABS CTAs in slabs of 128.  LAYER 0 single, 1 double; a pair's moments
+// (image_moments.cuh) stay in registers over all its nodes and are assembled
+// once.  Bound by the FP64 pipe (about 150 operations per node, 12 nodes per
+// accepted sub-triangle).  With the generated straight-line blocks evaluated
+// per node and one CTA per chunk it moved 50 GB of spills on a 1,702-triangle
+// fault with 301 targets (112 ms, 82 % of the call): the whole call 206 -> 34
+// ms, 24 uneven faults in one pass (24,000 triangles) 378 -> 42 ms.
+template <int LAYER, bool STR>
+__global__ void __launch_bounds__(128, 2)
 k_hs_store(const HsStoreArgs a, const int* __restrict__ chunk_leaf, const int* __restrict__ chunk_e0,
            double* __restrict__ store) {
   const int li = chunk_leaf[blockIdx.x], e0 = chunk_e0[blockIdx.x];
@@ -362,9 +444,9 @@ k_hs_store(const HsStoreArgs a, const int* __restrict__ chunk_leaf, const int* _
   const int ne = min(HSS_PTS, tn - e0);
   const int nt = a.ntri[li];
   double* out = store + a.base[li];
-  Quad12 Q;
-  quad12(Q);
-  for (int q = threadIdx.x; q < ne * nt; q += blockDim.x) {
+  ImageConst cst;
+  image_const(a.lam, a.mu, cst);
+  for (int q = blockIdx.y * blockDim.x + threadIdx.x; q < ne * nt; q += gridDim.y * blockDim.x) {
     const int e = e0 + q / nt, t = q % nt;
     // triangle of near position t: the concatenated ranges of the paired boxes
     int tri = -1, pos = 0;
@@ -379,31 +461,46 @@ k_hs_store(const HsStoreArgs a, const int* __restrict__ chunk_leaf, const int* _
     if (tri < 0) continue;
     const double* xb = a.tgt + 3 * (size_t)(t0 + e);
     const double X[3] = {xb[0], xb[1], -xb[2]};
-    double acc[54];
-    for (int k = 0; k < 54; k++) acc[k] = 0.0;
-    if (a.points) {  // a particle: the kernel blocks at the point
-      const double* y = a.pts + 3 * (size_t)tri;
-      const double* nv = a.nrm + 3 * (size_t)tri;
-      if (a.dosl) mindlin_image_sl_blk(a.lam, a.mu, X[0], X[1], X[2], y[0], y[1], y[2], acc);
-      if (a.dodl) mindlin_image_dl_blk(a.lam, a.mu, X[0], X[1], X[2], y[0], y[1], y[2], nv[0], nv[1], nv[2], acc + 27);
-    } else {
-      hs_pair_blk(a.tri + 9 * (size_t)tri, a.nrm + 3 * (size_t)tri, X, a.dosl, a.dodl, a.lam, a.mu, Q, a.eps,
-                  a.ncap, acc);
-    }
-    double* o = out + ((size_t)e * nt + t) * a.K;
-    int w = 0;
-    for (int layer = 0; layer < 2; layer++) {
-      if ((layer == 0 && !a.dosl) || (layer == 1 && !a.dodl)) continue;
-      for (int c = 0; c < 3; c++) {
-        const double* blk = acc + 27 * layer + 9 * c;
-        o[w] = blk[0]; o[w + 1] = blk[1]; o[w + 2] = blk[2];
-        w += 3;
-        if (a.dstr) {
-          for (int k = 0; k < 6; k++) o[w + k] = blk[3 + k];
-          w += 6;
-        }
+    const double* nv = a.nrm + 3 * (size_t)tri;
+    double acc[27];
+#pragma unroll
+    for (int k = 0; k < 27; k++) acc[k] = 0.0;
+    bool near_singular = false;
+    double add[27];
+    auto adapt = [&](const double* v) {
+      if (!near_singular)
+        for (int k = 0; k < 27; k++) add[k] = 0.0;
+      near_singular = true;
+      hs_adapt_blk<LAYER>(v, nv, X, cst, a.eps, a.ncap, add);
+    };
+    auto run = [&](auto& m) {
+      m.clear();
+      if (a.points) {  // a particle: the kernels at the point
+        ImageNode g;
+        image_node(X, a.pts + 3 * (size_t)tri, g);
+        m.add(g, 1.0);
+      } else {
+        hs_pair_moments(a.tri + 9 * (size_t)tri, X, m, adapt);
       }
+    };
+    if (LAYER == 0) {
+      ImageSL m;
+      run(m);
+      image_sl_assemble(m, cst, X[2], STR, acc);
+    } else {
+      ImageDL<STR> m;
+      run(m);
+      image_dl_assemble<STR>(m, cst, X[2], nv, acc);
     }
+    if (near_singular)
+#pragma unroll
+      for (int k = 0; k < 27; k++) acc[k] += add[k];
+    constexpr int KB = STR ? 9 : 3;
+    double* o = out + ((size_t)e * nt + t) * a.K + (LAYER == 1 && a.dosl ? 3 * KB : 0);
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+#pragma unroll
+      for (int k = 0; k < KB; k++) o[KB * c + k] = acc[9 * c + k];
   }
 }
 
@@ -436,8 +533,17 @@ int hs_take_ncap() {
 void launch_hs_store(cudaStream_t st, const HsStoreArgs& a, int nchunk, const int* chunk_leaf,
                      const int* chunk_e0, double* store) {
   if (nchunk <= 0) return;
-  k_hs_store<<<nchunk, 128, 0, st>>>(a, chunk_leaf, chunk_e0, store);
-  count_launch();
+  const dim3 grid(nchunk, HSS_SLABS);
+  if (a.dosl) {
+    if (a.dstr) k_hs_store<0, true><<<grid, 128, 0, st>>>(a, chunk_leaf, chunk_e0, store);
+    else k_hs_store<0, false><<<grid, 128, 0, st>>>(a, chunk_leaf, chunk_e0, store);
+    count_launch();
+  }
+  if (a.dodl) {
+    if (a.dstr) k_hs_store<1, true><<<grid, 128, 0, st>>>(a, chunk_leaf, chunk_e0, store);
+    else k_hs_store<1, false><<<grid, 128, 0, st>>>(a, chunk_leaf, chunk_e0, store);
+    count_launch();
+  }
   EFMM_CUDA_TRY(cudaGetLastError());
 }
 

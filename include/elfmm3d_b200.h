@@ -361,6 +361,14 @@ int efmm_pair_eval_host(double rlam, double rmu, const double *tri, const double
 int efmm_mindlin_image_kernel(int layer, double lam, double mu, const double *x, const double *s,
                               const double *nrm, double *out);
 
+/* The same kernels in the moment form the image near field integrates on the
+ * device, evaluated on the host: the responses at x of nnode nodes s
+ * (nnode,3) with weights w, out[27] as above (strain 0: displacements only,
+ * the strain entries of layer 1 zero).  For checks; no device is used.
+ * Returns 0, or 16 for a bad layer, nnode < 1 or a NULL pointer. */
+int efmm_mindlin_image_moments(int layer, int strain, double lam, double mu, const double *x, int nnode,
+                               const double *s, const double *w, const double *nrm, double *out);
+
 /* Device check of the tensor-core FP32 product (tcgen05.mma kind::tf32,
  * 3-term split) that carries the batched P2M: random A (K x M) and B
  * (N x K) against an FP64 host product; *rel = relative l2 error, *timeout
