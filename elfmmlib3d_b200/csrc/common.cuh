@@ -5,6 +5,7 @@
 #include <cstdio>
 
 #include "tri_integrals.cuh"
+#include "tri_edges.cuh"
 #include "harmonics.cuh"
 
 namespace efmm {

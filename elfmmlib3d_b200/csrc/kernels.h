@@ -21,7 +21,11 @@ struct NearArgs {
 
 void launch_tri_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
                      const double* sdl, int dosl, int dodl, TriRec* out);
-void launch_near_leaf(cudaStream_t st, const NearArgs& a);
+// edge records (tri_edges.cuh) with densities, for the one-right-hand-side
+// near field and the direct sum
+void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
+                          const double* sdl, int dosl, int dodl, TriEdge* out);
+void launch_near_leaf(cudaStream_t st, const NearArgs& a, const TriEdge* rec, int ntri);
 void launch_near_store(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
                        int dodisp, double* store);
 void launch_near_replay(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
@@ -76,7 +80,7 @@ void launch_near_split(cudaStream_t st, const NearArgs& a, int R, int NJ, int KB
                        const double* g1, const long long* sbase, const int* ntri, float* S, int ntask,
                        const BulkTask* tasks, const float* A, const long long* coff, double* C, int nsrc, int ntgt,
                        const long long* base, const double* store, int* err, cudaEvent_t* ev = nullptr);
-void launch_direct_all(cudaStream_t st, int ntri, const TriRec* trir, int nsrc, const double* src_pts,
+void launch_direct_all(cudaStream_t st, int ntri, const TriEdge* rec, int nsrc, const double* src_pts,
                        int ntgt, const double* tgt_pts, int dosl, int dodl, int dostrain_src,
                        int dostrain_tgt, double rlam, double rmu, double* u_src, double* e_src,
                        double* u_tgt, double* e_tgt);

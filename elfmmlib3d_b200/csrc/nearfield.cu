@@ -3,11 +3,9 @@
 // The near field of the reference (src/elfmm3dtria.f:968 _evalloc and the
 // ITER variant src/elfmm3dtria_iter_1.f:1240-1419) sums, for each evaluation
 // point, the exact single/double layer potential of every triangle in the
-// source boxes paired with the point's leaf box.  Here one CTA owns one leaf
-// box: the paired triangles stream through shared memory in tiles, each warp
-// takes one evaluation point against a tile (lanes split the triangles), and
-// the per-point partial sums are reduced with warp shuffles into shared-memory
-// accumulators that are written once at the end.
+// source boxes paired with the point's leaf box.
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 #include "tc_common.cuh"
@@ -42,9 +40,11 @@ __global__ void k_tri_prep(int n, const double* __restrict__ tri, const int* __r
 
 constexpr int NF_TILE = 64;    // triangles staged per tile
 constexpr int NF_WARPS = 4;    // warps per CTA
-constexpr int NF_MAXEP = 512;  // max evaluation points per leaf held in shared memory
 #ifndef NF_MINB
 #define NF_MINB 2               // resident CTAs per SM the register budget targets
+#endif
+#ifndef NL_MINB
+#define NL_MINB 3               // the same for the edge-integral kernels
 #endif
 
 __device__ __forceinline__ void stage_tile(TriRec* sm, const TriRec* __restrict__ g, int cnt) {
@@ -54,135 +54,194 @@ __device__ __forceinline__ void stage_tile(TriRec* sm, const TriRec* __restrict_
   for (int q = threadIdx.x; q < nv; q += blockDim.x) dst[q] = src[q];
 }
 
-// One CTA per leaf box.  Evaluation points of the leaf: its sources (sorted
-// centroids, self-aware) then its targets.  nb_start/nb_items: CSR of the
-// source boxes paired with the leaf; box_src_start/count give their triangle
-// ranges.  Outputs are ADDED to u (3/pt) and e (6/pt, xx yy zz xy xz yz).
-__global__ void __launch_bounds__(NF_WARPS * 32, NF_MINB)
-k_near_leaf(int nleaf, const int* __restrict__ leaves, const int* __restrict__ nb_start,
-            const int* __restrict__ nb_items, const int* __restrict__ box_src_start,
-            const int* __restrict__ box_src_count, const int* __restrict__ box_tgt_start,
-            const int* __restrict__ box_tgt_count, const TriRec* __restrict__ trir,
-            const double* __restrict__ src_pts, const double* __restrict__ tgt_pts, int dosl,
-            int dodl, int dostrain_src, int dostrain_tgt, int do_src, int do_tgt, double rlam,
-            double rmu, double* __restrict__ u_src, double* __restrict__ e_src,
-            double* __restrict__ u_tgt, double* __restrict__ e_tgt) {
-  __shared__ TriRec tile[NF_TILE];
-  __shared__ double acc[NF_MAXEP][9];
-  int leaf = leaves[blockIdx.x];
-  int s0 = box_src_start[leaf], sn = do_src ? box_src_count[leaf] : 0;
-  int t0 = box_tgt_start[leaf], tn = do_tgt ? box_tgt_count[leaf] : 0;
-  int nep = sn + tn;
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // process evaluation points in chunks of NF_MAXEP
-  for (int ep0 = 0; ep0 < nep; ep0 += NF_MAXEP) {
-    int nepc = min(NF_MAXEP, nep - ep0);
-    for (int q = threadIdx.x; q < nepc * 9; q += blockDim.x) (&acc[0][0])[q] = 0.0;
-    __syncthreads();
-    for (int b = nb_start[blockIdx.x]; b < nb_start[blockIdx.x + 1]; b++) {
-      int sb = nb_items[b];
-      int tr0 = box_src_start[sb], trn = box_src_count[sb];
-      for (int k0 = 0; k0 < trn; k0 += NF_TILE) {
-        int cnt = min(NF_TILE, trn - k0);
-        __syncthreads();
-        stage_tile(tile, trir + tr0 + k0, cnt);
-        __syncthreads();
-        for (int e = warp; e < nepc; e += NF_WARPS) {
-          int ep = ep0 + e;
-          bool is_src = ep < sn;
-          int pidx = is_src ? s0 + ep : t0 + (ep - sn);
-          const double* P = is_src ? src_pts + 3 * (size_t)pidx : tgt_pts + 3 * (size_t)pidx;
-          double X[3] = {P[0], P[1], P[2]};
-          bool dostrain = is_src ? dostrain_src : dostrain_tgt;
-          double u[3] = {0, 0, 0}, ee[6] = {0, 0, 0, 0, 0, 0};
-          for (int k = lane; k < cnt; k += 32) {
-            int tidx = tr0 + k0 + k;
-            bool self = is_src && (tidx == pidx);
-            const TriRec& r = tile[k];
-            pair_eval(r.f, r.ssl, r.sdl, dosl, dodl, dostrain, X, self, rlam, rmu, u, ee);
-          }
+// Edge records of the triangles (tri_edges.cuh) with their densities, in tree
+// order (perm: user position of each, or null).
+__global__ void k_tri_edge_prep(int n, const double* __restrict__ tri, const int* __restrict__ perm,
+                                const double* __restrict__ ssl, const double* __restrict__ sdl, int dosl, int dodl,
+                                TriEdge* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int j = perm ? perm[i] : i;
+  double t[9];
 #pragma unroll
-          for (int c = 0; c < 3; c++) u[c] = warp_sum(u[c]);
-          if (dostrain) {
+  for (int c = 0; c < 9; c++) t[c] = tri[9 * (size_t)j + c];
+  TriEdge r;
+  tri_edge_frame(t, r);
 #pragma unroll
-            for (int c = 0; c < 6; c++) ee[c] = warp_sum(ee[c]);
-          }
-          if (lane == 0) {
-            acc[e][0] += u[0]; acc[e][1] += u[1]; acc[e][2] += u[2];
-            if (dostrain)
-              for (int c = 0; c < 6; c++) acc[e][3 + c] += ee[c];
-          }
+  for (int c = 0; c < 3; c++) {
+    r.s[c] = dosl ? ssl[3 * (size_t)j + c] : 0.0;
+    r.b[c] = dodl ? sdl[3 * (size_t)j + c] : 0.0;
+  }
+  out[i] = r;
+}
+
+// Near field of one right-hand side.  Evaluation points of a leaf: its
+// sources (sorted centroids, self-aware) then its targets; the triangles of
+// its paired boxes stream through shared memory in tiles filled across boxes.
+// A CTA holds up to NL_THREADS points (equal chunks) and deals the tile's
+// triangles to S = NL_THREADS / points slices of threads: thread (point,
+// slice), so a leaf of 25 points fills 125 of 128 threads, every lane of a
+// slice reads the same record (broadcast), and the slices are added once per
+// leaf.  gridDim.y CTAs share a leaf's triangle list where there are too few
+// leaves for the chip.  Bound by the FP64 pipe: about 760 operations per pair
+// and layer (log1p, atan2 and six divisions among them).  One CTA per leaf
+// with one point per warp and lanes over the triangles of one box at a time,
+// on derivative tables (228 registers, half of the lanes idle), took 104 ms
+// on 327,680 triangles + 250,007 targets at iprec 2 (165 M pairs) and 2.66 ms
+// on 317 + 41 (about 20 leaves); this form 18.6 ms and 0.108 ms.  Registers
+// for 3 CTAs per SM: 2, 4 and 5 measured 23.6, 18.6 and 19.8 ms on the large
+// case, 1.23, 1.31 and 1.54 ms against 1.15 on 5,120 + 1,000.
+// Outputs are ADDED to u (3/pt) and e (6/pt, xx yy zz xy xz yz).
+constexpr int NL_THREADS = 128, NL_TILE = 32, NL_STRIDE = 34;  // record stride (doubles) free of bank conflicts
+
+template <bool SL, bool DL>
+__global__ void __launch_bounds__(NL_THREADS, NL_MINB)
+k_near_leaf(const NearArgs a, const TriEdge* __restrict__ rec) {
+  __shared__ __align__(16) double tile[NL_TILE * NL_STRIDE];
+  __shared__ int tidx[NL_TILE];
+  const int li = blockIdx.x, leaf = a.leaves[li], tid = threadIdx.x;
+  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0;
+  const int t0 = a.box_tgt_start[leaf], tn = a.do_tgt ? a.box_tgt_count[leaf] : 0;
+  const int nep = sn + tn;
+  if (nep == 0) return;
+  const double al = (a.rlam + a.rmu) / (a.rlam + 2.0 * a.rmu), i2mu = 0.5 / a.rmu;
+  const int nb0 = a.nb_start[li], nb1 = a.nb_start[li + 1];
+  // this CTA's part of the leaf's triangle list
+  int lo = 0, hi = 0x7fffffff;
+  if (gridDim.y > 1) {
+    int tot = 0;
+    for (int b = nb0; b < nb1; b++) tot += a.box_src_count[a.nb_items[b]];
+    lo = (int)((long long)tot * blockIdx.y / gridDim.y);
+    hi = (int)((long long)tot * (blockIdx.y + 1) / gridDim.y);
+    if (lo >= hi) return;
+  }
+  const int nch = (nep + NL_THREADS - 1) / NL_THREADS, cs = (nep + nch - 1) / nch, S = NL_THREADS / cs;
+  for (int ep0 = 0; ep0 < nep; ep0 += cs) {
+    const int e = ep0 + tid % cs, sl = tid / cs;
+    const bool on = sl < S && e < nep;
+    const bool is_src = e < sn;
+    const int pidx = is_src ? s0 + e : t0 + (e - sn);
+    const bool str = is_src ? a.dostrain_src : a.dostrain_tgt;
+    double X[3] = {0, 0, 0};
+    if (on) {
+      const double* P = (is_src ? a.src_pts : a.tgt_pts) + 3 * (size_t)pidx;
+      X[0] = P[0]; X[1] = P[1]; X[2] = P[2];
+    }
+    double u[3] = {0, 0, 0}, ee[6] = {0, 0, 0, 0, 0, 0};
+    int pos = 0, b = nb0, k = 0;  // list position, box and triangle of the box to stage next
+    while (b < nb1 && pos < hi) {
+      __syncthreads();
+      int fill = 0;
+      while (b < nb1 && fill < NL_TILE && pos < hi) {
+        const int sb = a.nb_items[b], cnt = a.box_src_count[sb];
+        const int skip = min(max(lo - pos, 0), cnt - k);  // before this CTA's part
+        k += skip;
+        pos += skip;
+        const int m = min(min(NL_TILE - fill, cnt - k), hi - pos);
+        const int tr0 = a.box_src_start[sb] + k;
+        const double2* src = reinterpret_cast<const double2*>(rec + tr0);
+        for (int q = tid; q < 16 * m; q += NL_THREADS)
+          reinterpret_cast<double2*>(tile + (fill + q / 16) * NL_STRIDE)[q % 16] = src[q];
+        if (tid < m) tidx[fill + tid] = tr0 + tid;
+        fill += m;
+        k += m;
+        pos += m;
+        if (k >= cnt) {
+          b++;
+          k = 0;
         }
       }
+      __syncthreads();
+      if (on)
+        for (int t = sl; t < fill; t += S) {
+          const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + t * NL_STRIDE);
+          tri_edge_pair<SL, DL>(T, X, is_src && tidx[t] == pidx, str, al, i2mu, u, ee);
+        }
     }
+    // add the slices
+    static_assert(NL_TILE * NL_STRIDE >= 8 * NL_THREADS, "reduction space");
     __syncthreads();
-    for (int e = threadIdx.x; e < nepc; e += blockDim.x) {
-      int ep = ep0 + e;
-      bool is_src = ep < sn;
-      int pidx = is_src ? s0 + ep : t0 + (ep - sn);
-      double* U = is_src ? u_src : u_tgt;
-      double* E = is_src ? e_src : e_tgt;
-      U[3 * (size_t)pidx] += acc[e][0];
-      U[3 * (size_t)pidx + 1] += acc[e][1];
-      U[3 * (size_t)pidx + 2] += acc[e][2];
-      bool dostrain = is_src ? dostrain_src : dostrain_tgt;
-      if (dostrain)
-        for (int c = 0; c < 6; c++) E[6 * (size_t)pidx + c] += acc[e][3 + c];
+    double out[9] = {u[0], u[1], u[2], ee[0], ee[1], ee[2], ee[3], ee[4], ee[5]};
+    for (int c0 = 0; c0 < 9; c0 += 8) {  // 8 values at a time through the tile
+#pragma unroll
+      for (int c = 0; c < 8; c++)
+        if (on && c0 + c < 9) tile[c * NL_THREADS + tid] = c0 == 0 ? out[c] : out[8];
+      __syncthreads();
+      if (on && sl == 0)
+#pragma unroll
+        for (int c = 0; c < 8; c++)
+          if (c0 + c < 9) {
+            double v = 0.0;
+            for (int q = 0; q < S; q++) v += tile[c * NL_THREADS + q * cs + tid];
+            if (c0 == 0) out[c] = v;
+            else out[8] = v;
+          }
+      __syncthreads();
     }
-    __syncthreads();
+    if (on && sl == 0) {
+      double* U = (is_src ? a.u_src : a.u_tgt) + 3 * (size_t)pidx;
+      double* E = (is_src ? a.e_src : a.e_tgt) + 6 * (size_t)pidx;
+      if (gridDim.y > 1) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) atomicAdd(U + c, out[c]);
+        if (str)
+#pragma unroll
+          for (int c = 0; c < 6; c++) atomicAdd(E + c, out[3 + c]);
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; c++) U[c] += out[c];
+        if (str)
+#pragma unroll
+          for (int c = 0; c < 6; c++) E[c] += out[3 + c];
+      }
+    }
   }
 }
 
-// All-pairs direct sum (el3dtriadirecttarg, src/elfmm3dtria.f:1483): one warp
-// per evaluation point, all triangles streamed through shared memory.
-// Points [0, nsrc) are the centroids (self pair when the indices match),
-// [nsrc, nsrc+ntgt) the targets.  Outputs are overwritten.
-__global__ void __launch_bounds__(NF_WARPS * 32, NF_MINB)
-k_direct_all(int ntri, const TriRec* __restrict__ trir, int nsrc, const double* __restrict__ src_pts,
-             int ntgt, const double* __restrict__ tgt_pts, int dosl, int dodl, int dostrain_src,
-             int dostrain_tgt, double rlam, double rmu, double* __restrict__ u_src,
-             double* __restrict__ e_src, double* __restrict__ u_tgt, double* __restrict__ e_tgt) {
-  __shared__ TriRec tile[NF_TILE];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int ep = blockIdx.x * NF_WARPS + warp;
-  int nep = nsrc + ntgt;
-  bool active = ep < nep;
-  bool is_src = ep < nsrc;
-  int pidx = is_src ? ep : ep - nsrc;
+// All-pairs direct sum (el3dtriadirecttarg, src/elfmm3dtria.f:1483): one
+// thread per evaluation point, all triangles streamed through shared memory;
+// gridDim.y CTAs share the triangles of a block of points (outputs zeroed by
+// the launcher and added to).  Points [0, nsrc) are the centroids (self pair
+// when the indices match), [nsrc, nsrc + ntgt) the targets.
+template <bool SL, bool DL>
+__global__ void __launch_bounds__(NL_THREADS, NL_MINB)
+k_direct_all(int ntri, const TriEdge* __restrict__ rec, int nsrc, const double* __restrict__ src_pts, int ntgt,
+             const double* __restrict__ tgt_pts, int dostrain_src, int dostrain_tgt, double rlam, double rmu,
+             double* __restrict__ u_src, double* __restrict__ e_src, double* __restrict__ u_tgt,
+             double* __restrict__ e_tgt) {
+  __shared__ __align__(16) double tile[NL_TILE * NL_STRIDE];
+  const int tid = threadIdx.x, ep = blockIdx.x * NL_THREADS + tid;
+  const bool on = ep < nsrc + ntgt, is_src = ep < nsrc;
+  const int pidx = is_src ? ep : ep - nsrc;
+  const bool str = is_src ? dostrain_src : dostrain_tgt;
+  const double al = (rlam + rmu) / (rlam + 2.0 * rmu), i2mu = 0.5 / rmu;
   double X[3] = {0, 0, 0};
-  if (active) {
-    const double* P = is_src ? src_pts + 3 * (size_t)pidx : tgt_pts + 3 * (size_t)pidx;
+  if (on) {
+    const double* P = (is_src ? src_pts : tgt_pts) + 3 * (size_t)pidx;
     X[0] = P[0]; X[1] = P[1]; X[2] = P[2];
   }
-  bool dostrain = is_src ? dostrain_src : dostrain_tgt;
+  const int lo = (int)((long long)ntri * blockIdx.y / gridDim.y);
+  const int hi = (int)((long long)ntri * (blockIdx.y + 1) / gridDim.y);
   double u[3] = {0, 0, 0}, ee[6] = {0, 0, 0, 0, 0, 0};
-  for (int k0 = 0; k0 < ntri; k0 += NF_TILE) {
-    int cnt = min(NF_TILE, ntri - k0);
+  for (int k0 = lo; k0 < hi; k0 += NL_TILE) {
+    const int m = min(NL_TILE, hi - k0);
     __syncthreads();
-    stage_tile(tile, trir + k0, cnt);
+    const double2* src = reinterpret_cast<const double2*>(rec + k0);
+    for (int q = tid; q < 16 * m; q += NL_THREADS)
+      reinterpret_cast<double2*>(tile + (q / 16) * NL_STRIDE)[q % 16] = src[q];
     __syncthreads();
-    if (active) {
-      for (int k = lane; k < cnt; k += 32) {
-        bool self = is_src && (k0 + k == pidx);
-        const TriRec& r = tile[k];
-        pair_eval(r.f, r.ssl, r.sdl, dosl, dodl, dostrain, X, self, rlam, rmu, u, ee);
+    if (on)
+      for (int t = 0; t < m; t++) {
+        const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + t * NL_STRIDE);
+        tri_edge_pair<SL, DL>(T, X, is_src && k0 + t == pidx, str, al, i2mu, u, ee);
       }
-    }
   }
-  if (!active) return;
-#pragma unroll
-  for (int c = 0; c < 3; c++) u[c] = warp_sum(u[c]);
-#pragma unroll
-  for (int c = 0; c < 6; c++) ee[c] = warp_sum(ee[c]);
-  if (lane == 0) {
-    double* U = is_src ? u_src : u_tgt;
-    double* E = is_src ? e_src : e_tgt;
-    U[3 * (size_t)pidx] = u[0];
-    U[3 * (size_t)pidx + 1] = u[1];
-    U[3 * (size_t)pidx + 2] = u[2];
-    if (dostrain)
-      for (int c = 0; c < 6; c++) E[6 * (size_t)pidx + c] = ee[c];
-  }
+  if (!on) return;
+  double* U = (is_src ? u_src : u_tgt) + 3 * (size_t)pidx;
+  double* E = (is_src ? e_src : e_tgt) + 6 * (size_t)pidx;
+  for (int c = 0; c < 3; c++) atomicAdd(U + c, u[c]);
+  if (str)
+    for (int c = 0; c < 6; c++) atomicAdd(E + c, ee[c]);
 }
 
 // ITER mode, first call: compute and store the unit-density response blocks
@@ -829,13 +888,31 @@ void launch_tri_prep(cudaStream_t st, int n, const double* tri, const int* perm,
   k_tri_prep<<<(n + 127) / 128, 128, 0, st>>>(n, tri, perm, ssl, sdl, dosl, dodl, out); count_launch();
 }
 
-void launch_near_leaf(cudaStream_t st, const NearArgs& a) {
+void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
+                          const double* sdl, int dosl, int dodl, TriEdge* out) {
+  if (n <= 0) return;
+  k_tri_edge_prep<<<(n + 127) / 128, 128, 0, st>>>(n, tri, perm, ssl, sdl, dosl, dodl, out); count_launch();
+}
+
+// CTAs per leaf (or block of points) so that a small grid still covers the
+// chip about three times (3 CTAs of 128 threads per SM, 148 SMs), but no
+// CTA of fewer than about 16 triangles.
+static int near_split(int nblocks, int ntri) {
+  const int want = (3 * 3 * 148 + nblocks - 1) / nblocks;
+  return std::max(1, std::min({want, (ntri + 15) / 16, 64}));
+}
+
+void launch_near_leaf(cudaStream_t st, const NearArgs& a, const TriEdge* rec, int ntri) {
   if (a.nleaf <= 0) return;
-  k_near_leaf<<<a.nleaf, NF_WARPS * 32, 0, st>>>(
-      a.nleaf, a.leaves, a.nb_start, a.nb_items, a.box_src_start, a.box_src_count,
-      a.box_tgt_start, a.box_tgt_count, a.trir, a.src_pts, a.tgt_pts, a.dosl, a.dodl,
-      a.dostrain_src, a.dostrain_tgt, a.do_src, a.do_tgt, a.rlam, a.rmu, a.u_src, a.e_src,
-      a.u_tgt, a.e_tgt); count_launch();
+  // a leaf's list rarely holds more than 9 of the leaves of a surface's share
+  const dim3 grid(a.nleaf, near_split(a.nleaf, std::min(ntri, 9 * (ntri / a.nleaf + 1))));
+  if (a.dosl && a.dodl)
+    k_near_leaf<true, true><<<grid, NL_THREADS, 0, st>>>(a, rec);
+  else if (a.dosl)
+    k_near_leaf<true, false><<<grid, NL_THREADS, 0, st>>>(a, rec);
+  else
+    k_near_leaf<false, true><<<grid, NL_THREADS, 0, st>>>(a, rec);
+  count_launch();
 }
 
 void launch_near_store(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
@@ -899,15 +976,32 @@ void launch_near_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int
   EFMM_CUDA_TRY(cudaGetLastError());
 }
 
-void launch_direct_all(cudaStream_t st, int ntri, const TriRec* trir, int nsrc, const double* src_pts,
-                       int ntgt, const double* tgt_pts, int dosl, int dodl, int dostrain_src,
-                       int dostrain_tgt, double rlam, double rmu, double* u_src, double* e_src,
-                       double* u_tgt, double* e_tgt) {
-  int nep = nsrc + ntgt;
+void launch_direct_all(cudaStream_t st, int ntri, const TriEdge* rec, int nsrc, const double* src_pts, int ntgt,
+                       const double* tgt_pts, int dosl, int dodl, int dostrain_src, int dostrain_tgt, double rlam,
+                       double rmu, double* u_src, double* e_src, double* u_tgt, double* e_tgt) {
+  const int nep = nsrc + ntgt;
   if (nep <= 0) return;
-  k_direct_all<<<(nep + NF_WARPS - 1) / NF_WARPS, NF_WARPS * 32, 0, st>>>(
-      ntri, trir, nsrc, src_pts, ntgt, tgt_pts, dosl, dodl, dostrain_src, dostrain_tgt, rlam, rmu,
-      u_src, e_src, u_tgt, e_tgt); count_launch();
+  if (nsrc > 0) {
+    EFMM_CUDA_TRY(cudaMemsetAsync(u_src, 0, 24 * (size_t)nsrc, st));
+    EFMM_CUDA_TRY(cudaMemsetAsync(e_src, 0, 48 * (size_t)nsrc, st));
+  }
+  if (ntgt > 0) {
+    EFMM_CUDA_TRY(cudaMemsetAsync(u_tgt, 0, 24 * (size_t)ntgt, st));
+    EFMM_CUDA_TRY(cudaMemsetAsync(e_tgt, 0, 48 * (size_t)ntgt, st));
+  }
+  const int nb = (nep + NL_THREADS - 1) / NL_THREADS;
+  const dim3 grid(nb, near_split(nb, ntri));
+  auto go = [&](auto kern) {
+    kern<<<grid, NL_THREADS, 0, st>>>(ntri, rec, nsrc, src_pts, ntgt, tgt_pts, dostrain_src, dostrain_tgt, rlam, rmu,
+                                      u_src, e_src, u_tgt, e_tgt);
+  };
+  if (dosl && dodl)
+    go(k_direct_all<true, true>);
+  else if (dosl)
+    go(k_direct_all<true, false>);
+  else
+    go(k_direct_all<false, true>);
+  count_launch();
 }
 
 }  // namespace efmm

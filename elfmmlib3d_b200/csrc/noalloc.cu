@@ -7,7 +7,7 @@
 // acceptable.  For them efmm_direct_noalloc evaluates the same O(N^2) analytic
 // direct sum as el3dtriadirecttarg_, with the caller providing inputs and
 // outputs in device memory and all intermediate data held in fixed-size
-// scratch arrays at file scope below.  Those arrays (about 11 MB) stay on a GPU
+// scratch arrays at file scope below.  Those arrays (about 13 MB) stay on a GPU
 // for the life of the process once this file's module is loaded there.  Under
 // CUDA's lazy module loading (the default since CUDA 12) that happens at the
 // first call on the device, which therefore must come before the caller's pool
@@ -23,7 +23,7 @@ constexpr int NOALLOC_MAX_PTS = 65536;  // evaluation points per call (centroids
 
 // Scratch shared by every call on a device; it keeps the last call's
 // contents.  Every entry a call reads is written earlier in the same call.
-static __device__ __align__(256) TriRec g_noalloc_tri[NOALLOC_MAX_TRI];
+static __device__ __align__(256) TriEdge g_noalloc_tri[NOALLOC_MAX_TRI];
 static __device__ __align__(256) double g_noalloc_u[3 * NOALLOC_MAX_PTS];
 static __device__ __align__(256) double g_noalloc_e[6 * NOALLOC_MAX_PTS];
 
@@ -33,7 +33,7 @@ static __device__ __align__(256) double g_noalloc_e[6 * NOALLOC_MAX_PTS];
 // belong to the device's primary context: after cudaDeviceReset they are
 // stale, and the entry point must not be used again in that process.
 struct NoallocPtrs {
-  TriRec* tri;
+  TriEdge* tri;
   double* u;
   double* e;
   bool ready;
@@ -108,7 +108,7 @@ extern "C" int efmm_direct_noalloc(double rlam, double rmu, int n, const double*
   int do_src = (u_src || e_src) ? n : 0;
   int do_tgt = (nt > 0 && (u_tgt || e_tgt)) ? nt : 0;
   try {
-    launch_tri_prep(st, n, tri, nullptr, ssl, sdl, dosl, dodl, S.tri);
+    launch_tri_edge_prep(st, n, tri, nullptr, ssl, sdl, dosl, dodl, S.tri);
     launch_direct_all(st, n, S.tri, do_src, src, do_tgt, tgt, dosl, dodl, e_src ? 1 : 0,
                       e_tgt ? 1 : 0, rlam, rmu, S.u, S.e, S.u + 3 * (size_t)n, S.e + 6 * (size_t)n);
     if (do_src) {

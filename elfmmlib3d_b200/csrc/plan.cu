@@ -1198,8 +1198,8 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
   EFMM_CUDA_TRY(cudaEventRecord(ev_[6], st_));
   // near field
   trir_.resize(n);
-  if (mode != 2 && !points_)  // the stored operator replaces the triangle records
-    launch_tri_prep(st_, n, tri_s_.get(), nullptr, ssl_s_.get(), sdl_s_.get(), dosl, dodl, trir_.get());
+  if (mode == 1 && !points_)  // the stored operator replaces the triangle records
+    launch_tri_prep(st_, n, tri_s_.get(), nullptr, nullptr, nullptr, 0, 0, trir_.get());
   NearArgs na;
   na.nleaf = nnear_;
   na.leaves = near_leaves_.get(); na.nb_start = near_start_.get(); na.nb_items = near_items_.get();
@@ -1216,7 +1216,9 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     na.part_dl = dodl ? sdl_s_.get() : nullptr;
     launch_near_points(st_, na, nrm_s_.get(), rlam, rmu);
   } else if (mode == 0) {
-    launch_near_leaf(st_, na);
+    tedge_.resize(n);
+    launch_tri_edge_prep(st_, n, tri_s_.get(), nullptr, ssl_s_.get(), sdl_s_.get(), dosl, dodl, tedge_.get());
+    launch_near_leaf(st_, na, tedge_.get(), n);
   } else {
     // stored operator rows carry displacement and (if any output wants it) strain
     NearArgs sa = na;
@@ -2098,8 +2100,8 @@ int Plan::evaluate_direct(double rlam, double rmu, const double* d_ssl, const do
     timings.total = timings.near;
     return IER_OK;
   }
-  trir_.resize(n);
-  launch_tri_prep(st_, n, tri_u_.get(), nullptr, d_ssl, d_sdl, dosl, dodl, trir_.get());
+  tedge_.resize(n);
+  launch_tri_edge_prep(st_, n, tri_u_.get(), nullptr, d_ssl, d_sdl, dosl, dodl, tedge_.get());
   u_s_.resize(3 * (size_t)n);
   e_s_.resize(6 * (size_t)n);
   ut_s_.resize(3 * (size_t)std::max(nt, 1));
@@ -2112,7 +2114,7 @@ int Plan::evaluate_direct(double rlam, double rmu, const double* d_ssl, const do
   int do_tgt = (nt > 0 && (d_u_tgt || d_e_tgt)) ? nt : 0;
   const int ns = nsub > 0 ? std::min(nsub, n) : n;
   EFMM_CUDA_TRY(cudaEventRecord(ev_[0], st_));
-  launch_direct_all(st_, n, trir_.get(), do_src, src_u_.get(), do_tgt, tgt_u_.get(), dosl, dodl,
+  launch_direct_all(st_, n, tedge_.get(), do_src, src_u_.get(), do_tgt, tgt_u_.get(), dosl, dodl,
                     d_e_src ? 1 : 0, d_e_tgt ? 1 : 0, rlam, rmu, u_s_.get(), e_s_.get(), ut_s_.get(),
                     et_s_.get());
   EFMM_CUDA_TRY(cudaEventRecord(ev_[1], st_));

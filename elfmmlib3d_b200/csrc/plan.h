@@ -430,6 +430,7 @@ class Plan {
   DevBuf<double> mpole_, local_;
   DevBuf<double> ssl_s_, sdl_s_, u_s_, e_s_, ut_s_, et_s_;
   DevBuf<TriRec> trir_;
+  DevBuf<TriEdge> tedge_;
   OpPool* ops_ = nullptr;
   cudaEvent_t ev_[10];
   int launches_ = 0;

@@ -451,7 +451,7 @@ float efmm_plan_elapsed(efmm_plan *plan, int a, int b);
  * tri (n,3,3), src (n,3), ssl/sdl (n,3; NULL disables a layer), tgt (nt,3);
  * outputs u_src (n,3), e_src (n,3,3), u_tgt (nt,3), e_tgt (nt,3,3), NULL
  * disables one.  Intermediates live in fixed file-scope device arrays
- * (about 11 MB per GPU, held until exit once loaded): at most 32768
+ * (about 13 MB per GPU, held until exit once loaded): at most 32768
  * triangles and 65536 evaluation points (n + nt) per call; larger sizes
  * return 16 with a message on stderr.  Enqueues on `stream` (a cudaStream_t,
  * NULL = legacy default stream) and returns.  The first call on a device
