@@ -4,7 +4,6 @@
 #include <cstdint>
 #include <cstdio>
 
-#include "tri_integrals.cuh"
 #include "tri_edges.cuh"
 #include "harmonics.cuh"
 
@@ -52,16 +51,6 @@ __host__ __device__ constexpr void quad12(Quad12& q) {
     q.w[k] = w3;
   }
 }
-
-// Per-triangle record used by the near-field kernels (tree order).
-// 24 doubles = 192 bytes, 16-byte aligned for vector loads.
-struct __align__(16) TriRec {
-  TriFrame f;        // 16 doubles
-  double ssl[3];     // single-layer density in the triangle frame
-  double sdl[3];     // double-layer density in the triangle frame
-  double pad[2];
-};
-static_assert(sizeof(TriRec) == 192, "TriRec layout");
 
 // Number of this library's kernels launched so far (all devices, all plans).
 // Raise a kernel's dynamic shared-memory limit to at least `bytes`, never

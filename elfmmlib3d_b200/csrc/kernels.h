@@ -6,11 +6,23 @@
 
 namespace efmm {
 
+// Work item of the one-right-hand-side near field: evaluation points
+// [e0, e0 + ne) of near leaf li against cnt triangles of its list from
+// offset k0 of its range r0; shared: other items hold more of the leaf's
+// triangles for the same points (outputs added atomically).
+struct NearTask {
+  int li, e0, ne, r0, k0, cnt, shared;
+};
+
 struct NearArgs {
   int nleaf;
   const int *leaves, *nb_start, *nb_items;
+  // the near triangles of leaf i in list order as ranges (first, count),
+  // rng_start[i] .. rng_start[i + 1]
+  const int* rng_start;
+  const int2* rng;
   const int *box_src_start, *box_src_count, *box_tgt_start, *box_tgt_count;
-  const TriRec* trir;
+  const TriEdge* rec;  // edge records of the triangles, tree order
   const double *src_pts, *tgt_pts;
   int dosl, dodl, dostrain_src, dostrain_tgt, do_src, do_tgt;
   double rlam, rmu;
@@ -19,25 +31,26 @@ struct NearArgs {
   const double* part_dl = nullptr;
 };
 
-void launch_tri_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
-                     const double* sdl, int dosl, int dodl, TriRec* out);
-// edge records (tri_edges.cuh) with densities, for the one-right-hand-side
-// near field and the direct sum
-void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
-                          const double* sdl, int dosl, int dodl, TriEdge* out);
-void launch_near_leaf(cudaStream_t st, const NearArgs& a, const TriEdge* rec, int ntri);
+// Edge records (tri_edges.cuh), with the densities that the one-right-hand-side
+// near field and the direct sum contract.
+void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const double* ssl, const double* sdl, int dosl,
+                          int dodl, TriEdge* out, int R = 1, int r = 0);
+void launch_near_leaf(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks);
+constexpr int NEAR_TASK_PTS = 128;  // evaluation points of a work item, at most
 void launch_near_store(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
-                       int dodisp, double* store);
+                       double* store);
 void launch_near_replay(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
                         int dodisp, const double* ssl, const double* sdl, const double* store);
-// R <= 64 right-hand sides; densities (ntri_all, 3, R) tree order, outputs
-// (R, nsrc or ntgt, 3 or 6) tree order, ADDED to.  With store != NULL the
-// pair blocks come from the ITER store (per leaf at sbase, sntri near
-// triangles) instead of being computed.
-void launch_near_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int* chunk_leaf,
-                       const int* chunk_e0, int R, int dostrain, const double* ssl, const double* sdl,
-                       int ntri_all, int nsrc, int ntgt, const long long* sbase = nullptr,
-                       const int* sntri = nullptr, const double* store = nullptr);
+// R <= 64 right-hand sides; densities (n, 3, R) tree order, outputs (R, nsrc
+// or ntgt, 3 or 6) tree order, ADDED to.  Items of at most NEAR_BATCH_PTS points.
+constexpr int NEAR_BATCH_PTS = 8;
+void launch_near_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R, int dostrain,
+                       const double* ssl, const double* sdl, int nsrc, int ntgt);
+// The same with the pair blocks of the ITER store (per leaf at sbase, sntri
+// near triangles), over chunks of 8 evaluation points.
+void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int* chunk_leaf,
+                              const int* chunk_e0, int R, int dostrain, const double* ssl, const double* sdl,
+                              int nsrc, int ntgt, const long long* sbase, const int* sntri, const double* store);
 // Mixed-precision replay of the stored near field on the tensor cores: the
 // FP64 store converted once to FP32 in the product layout (per leaf at the
 // store's offsets: A[NJ t + j][KB e + c], lda = KB x points, self pairs

@@ -12,156 +12,101 @@
 
 namespace efmm {
 
-// Build the per-triangle frame records in tree order and rotate the densities
-// into each triangle frame.
-__global__ void k_tri_prep(int n, const double* __restrict__ tri, const int* __restrict__ perm,
-                           const double* __restrict__ ssl, const double* __restrict__ sdl,
-                           int dosl, int dodl, TriRec* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  int j = perm ? perm[i] : i;
-  double t[9];
-#pragma unroll
-  for (int c = 0; c < 9; c++) t[c] = tri[9 * (size_t)j + c];
-  TriRec r;
-  tri_frame(t, r.f);
-  double a[3] = {0, 0, 0}, b[3] = {0, 0, 0};
-  if (dosl) { a[0] = ssl[3 * (size_t)j]; a[1] = ssl[3 * (size_t)j + 1]; a[2] = ssl[3 * (size_t)j + 2]; }
-  if (dodl) { b[0] = sdl[3 * (size_t)j]; b[1] = sdl[3 * (size_t)j + 1]; b[2] = sdl[3 * (size_t)j + 2]; }
-  const double* ax[3] = {r.f.e1, r.f.e2, r.f.e3};
-#pragma unroll
-  for (int c = 0; c < 3; c++) {
-    r.ssl[c] = ax[c][0] * a[0] + ax[c][1] * a[1] + ax[c][2] * a[2];
-    r.sdl[c] = ax[c][0] * b[0] + ax[c][1] * b[1] + ax[c][2] * b[2];
-  }
-  r.pad[0] = r.pad[1] = 0.0;
-  out[i] = r;
-}
+constexpr int NL_MINB = 3;  // resident CTAs per SM the edge-integral kernels' register budget targets
 
-constexpr int NF_TILE = 64;    // triangles staged per tile
-constexpr int NF_WARPS = 4;    // warps per CTA
-#ifndef NF_MINB
-#define NF_MINB 2               // resident CTAs per SM the register budget targets
-#endif
-#ifndef NL_MINB
-#define NL_MINB 3               // the same for the edge-integral kernels
-#endif
-
-__device__ __forceinline__ void stage_tile(TriRec* sm, const TriRec* __restrict__ g, int cnt) {
-  const double2* src = reinterpret_cast<const double2*>(g);
-  double2* dst = reinterpret_cast<double2*>(sm);
-  int nv = cnt * (int)(sizeof(TriRec) / sizeof(double2));
-  for (int q = threadIdx.x; q < nv; q += blockDim.x) dst[q] = src[q];
-}
-
-// Edge records of the triangles (tri_edges.cuh) with their densities, in tree
-// order (perm: user position of each, or null).
-__global__ void k_tri_edge_prep(int n, const double* __restrict__ tri, const int* __restrict__ perm,
-                                const double* __restrict__ ssl, const double* __restrict__ sdl, int dosl, int dodl,
+// Edge records of the triangles (tri_edges.cuh) with the densities of
+// right-hand side r0 of R (innermost).
+__global__ void k_tri_edge_prep(int n, const double* __restrict__ tri, const double* __restrict__ ssl,
+                                const double* __restrict__ sdl, int dosl, int dodl, int R, int r0,
                                 TriEdge* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const int j = perm ? perm[i] : i;
   double t[9];
 #pragma unroll
-  for (int c = 0; c < 9; c++) t[c] = tri[9 * (size_t)j + c];
+  for (int c = 0; c < 9; c++) t[c] = tri[9 * (size_t)i + c];
   TriEdge r;
   tri_edge_frame(t, r);
 #pragma unroll
   for (int c = 0; c < 3; c++) {
-    r.s[c] = dosl ? ssl[3 * (size_t)j + c] : 0.0;
-    r.b[c] = dodl ? sdl[3 * (size_t)j + c] : 0.0;
+    r.s[c] = dosl ? ssl[(3 * (size_t)i + c) * R + r0] : 0.0;
+    r.b[c] = dodl ? sdl[(3 * (size_t)i + c) * R + r0] : 0.0;
   }
   out[i] = r;
 }
 
 // Near field of one right-hand side.  Evaluation points of a leaf: its
-// sources (sorted centroids, self-aware) then its targets; the triangles of
-// its paired boxes stream through shared memory in tiles filled across boxes.
-// A CTA holds up to NL_THREADS points (equal chunks) and deals the tile's
-// triangles to S = NL_THREADS / points slices of threads: thread (point,
-// slice), so a leaf of 25 points fills 125 of 128 threads, every lane of a
-// slice reads the same record (broadcast), and the slices are added once per
-// leaf.  gridDim.y CTAs share a leaf's triangle list where there are too few
-// leaves for the chip.  Bound by the FP64 pipe: about 760 operations per pair
-// and layer (log1p, atan2 and six divisions among them).  One CTA per leaf
-// with one point per warp and lanes over the triangles of one box at a time,
-// on derivative tables (228 registers, half of the lanes idle), took 104 ms
-// on 327,680 triangles + 250,007 targets at iprec 2 (165 M pairs) and 2.66 ms
-// on 317 + 41 (about 20 leaves); this form 18.6 ms and 0.108 ms.  Registers
-// for 3 CTAs per SM: 2, 4 and 5 measured 23.6, 18.6 and 19.8 ms on the large
-// case, 1.23, 1.31 and 1.54 ms against 1.15 on 5,120 + 1,000.
+// sources (sorted centroids, self-aware) then its targets; a work item is a
+// few hundred to a few thousand pairs of one leaf (NearTask, the largest
+// first), its triangles stream through shared memory in tiles.  The tile's
+// triangles are dealt to S = NL_THREADS / points slices of threads: thread
+// (point, slice), so 25 points fill 125 of 128 threads, every lane of a slice
+// reads the same record (broadcast), and the slices are added once per item.
+// Bound by the FP64 pipe: about 760 operations per pair and layer (log1p,
+// atan2 and six divisions among them).  One CTA per leaf with one point per
+// warp and lanes over the triangles of one box at a time, on derivative
+// tables (228 registers, half of the lanes idle), took 104 ms on 327,680
+// triangles + 250,007 targets at iprec 2 (165 M pairs) and 2.66 ms on 317 + 41
+// (about 20 leaves); this form 18.3 ms and 0.058 ms.  Items instead of
+// whole leaves matter where a few leaves hold most pairs (a coarse target
+// leaf beside hundreds of fine source boxes): whole leaves took 12.5 ms
+// against 6.0 on 81,920 triangles + 62,501 shell targets (55 M pairs).
+// Registers for 3 CTAs per SM: 2, 4 and 5 measured 23.6, 18.6 and 19.8 ms on
+// the large case, 1.23, 1.31 and 1.54 ms against 1.15 on 5,120 + 1,000.
 // Outputs are ADDED to u (3/pt) and e (6/pt, xx yy zz xy xz yz).
-constexpr int NL_THREADS = 128, NL_TILE = 32, NL_STRIDE = 34;  // record stride (doubles) free of bank conflicts
+constexpr int NL_THREADS = NEAR_TASK_PTS, NL_TILE = 32, NL_STRIDE = 34;  // record stride (doubles) free of bank conflicts
 
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(NL_THREADS, NL_MINB)
-k_near_leaf(const NearArgs a, const TriEdge* __restrict__ rec) {
+k_near_leaf(const NearArgs a, const NearTask* __restrict__ tasks) {
   __shared__ __align__(16) double tile[NL_TILE * NL_STRIDE];
   __shared__ int tidx[NL_TILE];
-  const int li = blockIdx.x, leaf = a.leaves[li], tid = threadIdx.x;
-  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0;
-  const int t0 = a.box_tgt_start[leaf], tn = a.do_tgt ? a.box_tgt_count[leaf] : 0;
-  const int nep = sn + tn;
-  if (nep == 0) return;
+  const NearTask w = tasks[blockIdx.x];
+  const int leaf = a.leaves[w.li], tid = threadIdx.x;
+  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0, t0 = a.box_tgt_start[leaf];
   const double al = (a.rlam + a.rmu) / (a.rlam + 2.0 * a.rmu), i2mu = 0.5 / a.rmu;
-  const int nb0 = a.nb_start[li], nb1 = a.nb_start[li + 1];
-  // this CTA's part of the leaf's triangle list
-  int lo = 0, hi = 0x7fffffff;
-  if (gridDim.y > 1) {
-    int tot = 0;
-    for (int b = nb0; b < nb1; b++) tot += a.box_src_count[a.nb_items[b]];
-    lo = (int)((long long)tot * blockIdx.y / gridDim.y);
-    hi = (int)((long long)tot * (blockIdx.y + 1) / gridDim.y);
-    if (lo >= hi) return;
+  const int S = NL_THREADS / w.ne, sl = tid / w.ne, e = w.e0 + tid % w.ne;
+  const bool on = sl < S;
+  const bool is_src = e < sn;
+  const int pidx = is_src ? s0 + e : t0 + (e - sn);
+  const bool str = is_src ? a.dostrain_src : a.dostrain_tgt;
+  double X[3] = {0, 0, 0};
+  if (on) {
+    const double* P = (is_src ? a.src_pts : a.tgt_pts) + 3 * (size_t)pidx;
+    X[0] = P[0]; X[1] = P[1]; X[2] = P[2];
   }
-  const int nch = (nep + NL_THREADS - 1) / NL_THREADS, cs = (nep + nch - 1) / nch, S = NL_THREADS / cs;
-  for (int ep0 = 0; ep0 < nep; ep0 += cs) {
-    const int e = ep0 + tid % cs, sl = tid / cs;
-    const bool on = sl < S && e < nep;
-    const bool is_src = e < sn;
-    const int pidx = is_src ? s0 + e : t0 + (e - sn);
-    const bool str = is_src ? a.dostrain_src : a.dostrain_tgt;
-    double X[3] = {0, 0, 0};
-    if (on) {
-      const double* P = (is_src ? a.src_pts : a.tgt_pts) + 3 * (size_t)pidx;
-      X[0] = P[0]; X[1] = P[1]; X[2] = P[2];
-    }
-    double u[3] = {0, 0, 0}, ee[6] = {0, 0, 0, 0, 0, 0};
-    int pos = 0, b = nb0, k = 0;  // list position, box and triangle of the box to stage next
-    while (b < nb1 && pos < hi) {
-      __syncthreads();
-      int fill = 0;
-      while (b < nb1 && fill < NL_TILE && pos < hi) {
-        const int sb = a.nb_items[b], cnt = a.box_src_count[sb];
-        const int skip = min(max(lo - pos, 0), cnt - k);  // before this CTA's part
-        k += skip;
-        pos += skip;
-        const int m = min(min(NL_TILE - fill, cnt - k), hi - pos);
-        const int tr0 = a.box_src_start[sb] + k;
-        const double2* src = reinterpret_cast<const double2*>(rec + tr0);
-        for (int q = tid; q < 16 * m; q += NL_THREADS)
-          reinterpret_cast<double2*>(tile + (fill + q / 16) * NL_STRIDE)[q % 16] = src[q];
-        if (tid < m) tidx[fill + tid] = tr0 + tid;
-        fill += m;
-        k += m;
-        pos += m;
-        if (k >= cnt) {
-          b++;
-          k = 0;
-        }
-      }
-      __syncthreads();
-      if (on)
-        for (int t = sl; t < fill; t += S) {
-          const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + t * NL_STRIDE);
-          tri_edge_pair<SL, DL>(T, X, is_src && tidx[t] == pidx, str, al, i2mu, u, ee);
-        }
-    }
-    // add the slices
-    static_assert(NL_TILE * NL_STRIDE >= 8 * NL_THREADS, "reduction space");
+  double u[3] = {0, 0, 0}, ee[6] = {0, 0, 0, 0, 0, 0};
+  int left = w.cnt, b = w.r0, k = w.k0;  // range and triangle of the range to stage next
+  while (left > 0) {
     __syncthreads();
-    double out[9] = {u[0], u[1], u[2], ee[0], ee[1], ee[2], ee[3], ee[4], ee[5]};
+    int fill = 0;
+    while (left > 0 && fill < NL_TILE) {  // tiles fill across ranges
+      const int2 rg = a.rng[b];
+      const int m = min(min(NL_TILE - fill, rg.y - k), left);
+      const int tr0 = rg.x + k;
+      const double2* src = reinterpret_cast<const double2*>(a.rec + tr0);
+      for (int q = tid; q < 16 * m; q += NL_THREADS)
+        reinterpret_cast<double2*>(tile + (fill + q / 16) * NL_STRIDE)[q % 16] = src[q];
+      if (tid < m) tidx[fill + tid] = tr0 + tid;
+      fill += m;
+      left -= m;
+      k += m;
+      if (k >= rg.y) {
+        b++;
+        k = 0;
+      }
+    }
+    __syncthreads();
+    if (on)
+      for (int t = sl; t < fill; t += S) {
+        const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + t * NL_STRIDE);
+        tri_edge_pair<SL, DL>(T, X, is_src && tidx[t] == pidx, str, al, i2mu, u, ee);
+      }
+  }
+  // add the slices
+  static_assert(NL_TILE * NL_STRIDE >= 8 * NL_THREADS, "reduction space");
+  __syncthreads();
+  double out[9] = {u[0], u[1], u[2], ee[0], ee[1], ee[2], ee[3], ee[4], ee[5]};
+  if (S > 1)
     for (int c0 = 0; c0 < 9; c0 += 8) {  // 8 values at a time through the tile
 #pragma unroll
       for (int c = 0; c < 8; c++)
@@ -172,28 +117,27 @@ k_near_leaf(const NearArgs a, const TriEdge* __restrict__ rec) {
         for (int c = 0; c < 8; c++)
           if (c0 + c < 9) {
             double v = 0.0;
-            for (int q = 0; q < S; q++) v += tile[c * NL_THREADS + q * cs + tid];
+            for (int q = 0; q < S; q++) v += tile[c * NL_THREADS + q * w.ne + tid];
             if (c0 == 0) out[c] = v;
             else out[8] = v;
           }
       __syncthreads();
     }
-    if (on && sl == 0) {
-      double* U = (is_src ? a.u_src : a.u_tgt) + 3 * (size_t)pidx;
-      double* E = (is_src ? a.e_src : a.e_tgt) + 6 * (size_t)pidx;
-      if (gridDim.y > 1) {
+  if (on && sl == 0) {
+    double* U = (is_src ? a.u_src : a.u_tgt) + 3 * (size_t)pidx;
+    double* E = (is_src ? a.e_src : a.e_tgt) + 6 * (size_t)pidx;
+    if (w.shared) {
 #pragma unroll
-        for (int c = 0; c < 3; c++) atomicAdd(U + c, out[c]);
-        if (str)
+      for (int c = 0; c < 3; c++) atomicAdd(U + c, out[c]);
+      if (str)
 #pragma unroll
-          for (int c = 0; c < 6; c++) atomicAdd(E + c, out[3 + c]);
-      } else {
+        for (int c = 0; c < 6; c++) atomicAdd(E + c, out[3 + c]);
+    } else {
 #pragma unroll
-        for (int c = 0; c < 3; c++) U[c] += out[c];
-        if (str)
+      for (int c = 0; c < 3; c++) U[c] += out[c];
+      if (str)
 #pragma unroll
-          for (int c = 0; c < 6; c++) E[c] += out[3 + c];
-      }
+        for (int c = 0; c < 6; c++) E[c] += out[3 + c];
     }
   }
 }
@@ -247,40 +191,61 @@ k_direct_all(int ntri, const TriEdge* __restrict__ rec, int nsrc, const double* 
 // ITER mode, first call: compute and store the unit-density response blocks
 // of every near (point, triangle) pair of each leaf.  Layout per leaf:
 // [evaluation point][near triangle][K doubles], at base[leaf]; near triangles
-// are the concatenated source ranges of the leaf's paired boxes.
-__global__ void __launch_bounds__(NF_WARPS * 32, NF_MINB)
+// are the concatenated source ranges of the leaf's paired boxes.  Tiles of 64
+// triangles of one box, a warp per evaluation point (dealt over gridDim.y
+// CTAs), lanes over the tile.
+constexpr int NF_TILE = 64, NF_WARPS = 4;
+
+__device__ __forceinline__ void near_pair_blocks(const TriEdge& T, const double* X, bool self, int dosl, int dodl,
+                                                 int str, double al, double i2mu, double* out) {
+  if (str) {
+    if (dosl) {
+      tri_edge_blocks<0, true>(T, X, self, al, i2mu, out);
+      out += 27;
+    }
+    if (dodl) tri_edge_blocks<1, true>(T, X, self, al, i2mu, out);
+  } else {
+    if (dosl) {
+      tri_edge_blocks<0, false>(T, X, self, al, i2mu, out);
+      out += 9;
+    }
+    if (dodl) tri_edge_blocks<1, false>(T, X, self, al, i2mu, out);
+  }
+}
+
+__global__ void __launch_bounds__(NF_WARPS * 32, NL_MINB)
 k_near_store(const NearArgs a, const long long* __restrict__ base, const int* __restrict__ ntri,
-             int K, int dodisp, double* __restrict__ store) {
-  __shared__ TriRec tile[NF_TILE];
-  int leaf = a.leaves[blockIdx.x];
-  int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0;
-  int t0 = a.box_tgt_start[leaf], tn = a.do_tgt ? a.box_tgt_count[leaf] : 0;
-  int nep = sn + tn;
-  int nt = ntri[blockIdx.x];
+             int K, double* __restrict__ store) {
+  __shared__ __align__(16) double tile[NF_TILE * NL_STRIDE];
+  const int leaf = a.leaves[blockIdx.x];
+  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0;
+  const int t0 = a.box_tgt_start[leaf], tn = a.do_tgt ? a.box_tgt_count[leaf] : 0;
+  const int nep = sn + tn;
+  const int nt = ntri[blockIdx.x];
+  const double al = (a.rlam + a.rmu) / (a.rlam + 2.0 * a.rmu), i2mu = 0.5 / a.rmu;
   double* out = store + base[blockIdx.x];
-  int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int pos = 0;  // running index of the leaf's near triangles
   for (int b = a.nb_start[blockIdx.x]; b < a.nb_start[blockIdx.x + 1]; b++) {
-    int sb = a.nb_items[b];
-    int tr0 = a.box_src_start[sb], trn = a.box_src_count[sb];
+    const int sb = a.nb_items[b];
+    const int tr0 = a.box_src_start[sb], trn = a.box_src_count[sb];
     for (int k0 = 0; k0 < trn; k0 += NF_TILE) {
-      int cnt = min(NF_TILE, trn - k0);
+      const int cnt = min(NF_TILE, trn - k0);
       __syncthreads();
-      stage_tile(tile, a.trir + tr0 + k0, cnt);
+      const double2* src = reinterpret_cast<const double2*>(a.rec + tr0 + k0);
+      for (int q = threadIdx.x; q < 16 * cnt; q += NF_WARPS * 32)
+        reinterpret_cast<double2*>(tile + (q / 16) * NL_STRIDE)[q % 16] = src[q];
       __syncthreads();
-      for (int e = warp; e < nep; e += NF_WARPS) {
-        bool is_src = e < sn;
-        int pidx = is_src ? s0 + e : t0 + (e - sn);
+      for (int e = warp + NF_WARPS * blockIdx.y; e < nep; e += NF_WARPS * gridDim.y) {
+        const bool is_src = e < sn;
+        const int pidx = is_src ? s0 + e : t0 + (e - sn);
         const double* P = is_src ? a.src_pts + 3 * (size_t)pidx : a.tgt_pts + 3 * (size_t)pidx;
-        double X[3] = {P[0], P[1], P[2]};
-        bool dostrain = is_src ? a.dostrain_src : a.dostrain_tgt;
+        const double X[3] = {P[0], P[1], P[2]};
+        const int str = is_src ? a.dostrain_src : a.dostrain_tgt;
         for (int k = lane; k < cnt; k += 32) {
-          int tidx = tr0 + k0 + k;
-          bool self = is_src && (tidx == pidx);
-          double blk[54];
-          pair_blocks(tile[k].f, a.dosl, a.dodl, dodisp, dostrain, X, self, a.rlam, a.rmu, blk);
-          double* o = out + ((size_t)e * nt + (pos + k0 + k)) * K;
-          for (int q = 0; q < K; q++) o[q] = blk[q];
+          const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + k * NL_STRIDE);
+          near_pair_blocks(T, X, is_src && tr0 + k0 + k == pidx, a.dosl, a.dodl, str, al, i2mu,
+                           out + ((size_t)e * nt + (pos + k0 + k)) * K);
         }
       }
     }
@@ -352,40 +317,35 @@ k_near_replay(const NearArgs a, const long long* __restrict__ base, const int* _
 
 // Many right-hand sides at once (densities tree order, right-hand side
 // innermost: sigma[(tri * 3 + component) * R + r]).  The pair response to unit densities
-// (pair_blocks, as stored by the ITER mode) does not depend on the densities,
+// (tri_edge_blocks, as stored by the ITER mode) does not depend on the densities,
 // so it is computed once per (point, triangle) pair and contracted with all
 // R right-hand sides: per tile of NB_PTS points x NB_TRI triangles, phase 1
 // writes the pair blocks to shared memory (one pair per thread), phase 2 is a
 // small dense product  out[point][9][R] += block[point][tri][9 x 6] *
 // sigma[tri][6][R]  with the outputs held in registers (9 x RB per thread;
 // R <= 16 RB).  One CTA per (near leaf, chunk of NB_PTS evaluation points).
-constexpr int NB_PTS = 8, NB_TRI = 16, NB_THREADS = NB_PTS * NB_TRI;
+constexpr int NB_PTS = NEAR_BATCH_PTS, NB_TRI = 16, NB_THREADS = NB_PTS * NB_TRI;
 
-// REPLAY: the pair blocks are read from the stored near field (k_near_store
-// layout: per leaf at base[leaf], [point][near triangle][K]) instead of
-// computed -- the ITER store applied to many right-hand sides at once.
-template <int RB, bool REPLAY>
+template <int RB>
 __global__ void __launch_bounds__(NB_THREADS)
-k_near_batch(const NearArgs a, const int* __restrict__ chunk_leaf, const int* __restrict__ chunk_e0,
-             int R, int K, int dostrain, const double* __restrict__ ssl, const double* __restrict__ sdl,
-             int ntri_all, int nsrc, int ntgt, const long long* __restrict__ sbase, const int* __restrict__ sntri,
-             const double* __restrict__ store) {
+k_near_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R, int K, int dostrain,
+             const double* __restrict__ ssl, const double* __restrict__ sdl, int nsrc, int ntgt) {
   constexpr int RW = 16 * RB;  // right-hand sides held per tile
-  __shared__ TriRec tile[NB_TRI];
+  __shared__ __align__(16) double tile[NB_TRI * NL_STRIDE];
+  __shared__ int tidx[NB_TRI];
   extern __shared__ __align__(16) double nb_sm[];
   double* Bk = nb_sm;                            // [NB_PTS][NB_TRI][K]
   double* Sg = Bk + NB_PTS * NB_TRI * K;         // [NB_TRI][6][RW]
-  const int li = chunk_leaf[blockIdx.x], e0 = chunk_e0[blockIdx.x];
-  const int leaf = a.leaves[li];
-  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0;
-  const int t0 = a.box_tgt_start[leaf], tn = a.do_tgt ? a.box_tgt_count[leaf] : 0;
-  const int nep = sn + tn;
+  const NearTask w = tasks[blockIdx.x];
+  const int leaf = a.leaves[w.li];
+  const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0, t0 = a.box_tgt_start[leaf];
   const int tid = threadIdx.x;
   const int pp = tid / NB_TRI, tt = tid % NB_TRI;  // phase 1: (point, triangle)
   const int rr = tid % 16, pq = tid / 16;          // phase 2: (point, rhs lane)
+  const double al = (a.rlam + a.rmu) / (a.rlam + 2.0 * a.rmu), i2mu = 0.5 / a.rmu;
   // phase-1 point
-  const int e1 = e0 + pp;
-  const bool ok1 = e1 < nep;
+  const int e1 = w.e0 + pp;
+  const bool ok1 = pp < w.ne;
   const bool src1 = e1 < sn;
   const int pid1 = ok1 ? (src1 ? s0 + e1 : t0 + (e1 - sn)) : 0;
   double X[3] = {0, 0, 0};
@@ -398,75 +358,71 @@ k_near_batch(const NearArgs a, const int* __restrict__ chunk_leaf, const int* __
   for (int c = 0; c < 9; c++)
 #pragma unroll
     for (int k = 0; k < RB; k++) acc[c][k] = 0.0;
-  const int nl = a.dosl + a.dodl;
-  int pos = 0;  // running index of the leaf's near triangles (store layout)
-  for (int b = a.nb_start[li]; b < a.nb_start[li + 1]; b++) {
-    const int sb = a.nb_items[b];
-    const int tr0 = a.box_src_start[sb], trn = a.box_src_count[sb];
-    for (int k0 = 0; k0 < trn; k0 += NB_TRI) {
-      const int cnt = min(NB_TRI, trn - k0);
-      __syncthreads();
-      if (!REPLAY) stage_tile(tile, a.trir + tr0 + k0, cnt);
-      for (int q = tid; q < NB_TRI * 6 * RW; q += NB_THREADS) {
-        int t = q / (6 * RW), j = (q / RW) % 6, r = q % RW;
-        int layer = j / 3, d = j % 3;
-        double v = 0.0;
-        if (t < cnt && r < R && (layer == 0 ? a.dosl : a.dodl)) {
-          const double* sg = layer == 0 ? ssl : sdl;
-          v = sg[((size_t)(tr0 + k0 + t) * 3 + d) * R + r];
-        }
-        Sg[q] = v;
+  int left = w.cnt, b = w.r0, k = w.k0;  // range and triangle of the range to stage next
+  while (left > 0) {
+    __syncthreads();
+    int cnt = 0;
+    while (left > 0 && cnt < NB_TRI) {  // tiles fill across ranges
+      const int2 rg = a.rng[b];
+      const int m = min(min(NB_TRI - cnt, rg.y - k), left), tr0 = rg.x + k;
+      const double2* src = reinterpret_cast<const double2*>(a.rec + tr0);
+      for (int q = tid; q < 16 * m; q += NB_THREADS)
+        reinterpret_cast<double2*>(tile + (cnt + q / 16) * NL_STRIDE)[q % 16] = src[q];
+      if (tid < m) tidx[cnt + tid] = tr0 + tid;
+      cnt += m;
+      left -= m;
+      k += m;
+      if (k >= rg.y) {
+        b++;
+        k = 0;
       }
-      __syncthreads();
-      if (REPLAY) {
-        // the tile's blocks of the chunk's points: contiguous K-runs per point
-        const int nt = sntri[li];
-        const double* src = store + sbase[li];
-        for (int q = tid; q < NB_PTS * NB_TRI * K; q += NB_THREADS) {
-          const int pt = q / (NB_TRI * K), rem = q % (NB_TRI * K), t = rem / K, c = rem % K;
-          const int e = e0 + pt;
-          double v = 0.0;
-          if (e < nep && t < cnt) v = src[((size_t)e * nt + (pos + k0 + t)) * K + c];
-          Bk[q] = v;
-        }
+    }
+    __syncthreads();
+    for (int q = tid; q < NB_TRI * 6 * RW; q += NB_THREADS) {
+      const int t = q / (6 * RW), j = (q / RW) % 6, r = q % RW;
+      const int layer = j / 3, d = j % 3;
+      double v = 0.0;
+      if (t < cnt && r < R && (layer == 0 ? a.dosl : a.dodl)) {
+        const double* sg = layer == 0 ? ssl : sdl;
+        v = sg[((size_t)tidx[t] * 3 + d) * R + r];
+      }
+      Sg[q] = v;
+    }
+    {
+      double* o = Bk + (pp * NB_TRI + tt) * K;
+      if (ok1 && tt < cnt) {
+        const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + tt * NL_STRIDE);
+        near_pair_blocks(T, X, src1 && tidx[tt] == pid1, a.dosl, a.dodl, dostrain, al, i2mu, o);
       } else {
-        double* o = Bk + (pp * NB_TRI + tt) * K;
-        if (ok1 && tt < cnt) {
-          const int tidx = tr0 + k0 + tt;
-          pair_blocks(tile[tt].f, a.dosl, a.dodl, true, dostrain, X, src1 && tidx == pid1, a.rlam, a.rmu, o);
-        } else {
-          for (int q = 0; q < K; q++) o[q] = 0.0;
-        }
+        for (int q = 0; q < K; q++) o[q] = 0.0;
       }
-      __syncthreads();
-      for (int t = 0; t < cnt; t++) {
-        const double* Bt = Bk + (pq * NB_TRI + t) * K;
-        int w = 0;
-        for (int j = 0; j < 6; j++) {
-          if ((j < 3 && !a.dosl) || (j >= 3 && !a.dodl)) continue;
-          double sv[RB];
+    }
+    __syncthreads();
+    for (int t = 0; t < cnt; t++) {
+      const double* Bt = Bk + (pq * NB_TRI + t) * K;
+      int q0 = 0;
+      for (int j = 0; j < 6; j++) {
+        if ((j < 3 && !a.dosl) || (j >= 3 && !a.dodl)) continue;
+        double sv[RB];
 #pragma unroll
-          for (int k = 0; k < RB; k++) sv[k] = Sg[(t * 6 + j) * RW + rr + 16 * k];
+        for (int q = 0; q < RB; q++) sv[q] = Sg[(t * 6 + j) * RW + rr + 16 * q];
 #pragma unroll
-          for (int c = 0; c < 3; c++)
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-            for (int k = 0; k < RB; k++) acc[c][k] += Bt[w + c] * sv[k];
-          w += 3;
-          if (dostrain) {
+          for (int q = 0; q < RB; q++) acc[c][q] += Bt[q0 + c] * sv[q];
+        q0 += 3;
+        if (dostrain) {
 #pragma unroll
-            for (int c = 0; c < 6; c++)
+          for (int c = 0; c < 6; c++)
 #pragma unroll
-              for (int k = 0; k < RB; k++) acc[3 + c][k] += Bt[w + c] * sv[k];
-            w += 6;
-          }
+            for (int q = 0; q < RB; q++) acc[3 + c][q] += Bt[q0 + c] * sv[q];
+          q0 += 6;
         }
       }
     }
-    pos += trn;
   }
-  (void)nl;
-  const int e2 = e0 + pq;
-  if (e2 >= nep) return;
+  const int e2 = w.e0 + pq;
+  if (pq >= w.ne) return;
   const bool src2 = e2 < sn;
   const int pid2 = src2 ? s0 + e2 : t0 + (e2 - sn);
   const size_t np = src2 ? (size_t)nsrc : (size_t)ntgt;
@@ -476,12 +432,19 @@ k_near_batch(const NearArgs a, const int* __restrict__ chunk_leaf, const int* __
     const int r = rr + 16 * k;
     if (r >= R) continue;
     double* U = (src2 ? a.u_src : a.u_tgt) + 3 * (np * r + pid2);
+    double* E = (src2 ? a.e_src : a.e_tgt) + 6 * (np * r + pid2);
+    if (w.shared) {
 #pragma unroll
-    for (int c = 0; c < 3; c++) U[c] += acc[c][k];
-    if (ds2) {
-      double* E = (src2 ? a.e_src : a.e_tgt) + 6 * (np * r + pid2);
+      for (int c = 0; c < 3; c++) atomicAdd(U + c, acc[c][k]);
+      if (ds2)
 #pragma unroll
-      for (int c = 0; c < 6; c++) E[c] += acc[3 + c][k];
+        for (int c = 0; c < 6; c++) atomicAdd(E + c, acc[3 + c][k]);
+    } else {
+#pragma unroll
+      for (int c = 0; c < 3; c++) U[c] += acc[c][k];
+      if (ds2)
+#pragma unroll
+        for (int c = 0; c < 6; c++) E[c] += acc[3 + c][k];
     }
   }
 }
@@ -882,43 +845,27 @@ void launch_near_tc(cudaStream_t st, const NearArgs& a, int R, int NJ, int KB, c
 }
 
 // ---------------------------------------------------------------- launchers
-void launch_tri_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
-                     const double* sdl, int dosl, int dodl, TriRec* out) {
+void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const double* ssl, const double* sdl, int dosl,
+                          int dodl, TriEdge* out, int R, int r) {
   if (n <= 0) return;
-  k_tri_prep<<<(n + 127) / 128, 128, 0, st>>>(n, tri, perm, ssl, sdl, dosl, dodl, out); count_launch();
+  k_tri_edge_prep<<<(n + 127) / 128, 128, 0, st>>>(n, tri, ssl, sdl, dosl, dodl, R, r, out); count_launch();
 }
 
-void launch_tri_edge_prep(cudaStream_t st, int n, const double* tri, const int* perm, const double* ssl,
-                          const double* sdl, int dosl, int dodl, TriEdge* out) {
-  if (n <= 0) return;
-  k_tri_edge_prep<<<(n + 127) / 128, 128, 0, st>>>(n, tri, perm, ssl, sdl, dosl, dodl, out); count_launch();
-}
-
-// CTAs per leaf (or block of points) so that a small grid still covers the
-// chip about three times (3 CTAs of 128 threads per SM, 148 SMs), but no
-// CTA of fewer than about 16 triangles.
-static int near_split(int nblocks, int ntri) {
-  const int want = (3 * 3 * 148 + nblocks - 1) / nblocks;
-  return std::max(1, std::min({want, (ntri + 15) / 16, 64}));
-}
-
-void launch_near_leaf(cudaStream_t st, const NearArgs& a, const TriEdge* rec, int ntri) {
-  if (a.nleaf <= 0) return;
-  // a leaf's list rarely holds more than 9 of the leaves of a surface's share
-  const dim3 grid(a.nleaf, near_split(a.nleaf, std::min(ntri, 9 * (ntri / a.nleaf + 1))));
+void launch_near_leaf(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks) {
+  if (ntask <= 0) return;
   if (a.dosl && a.dodl)
-    k_near_leaf<true, true><<<grid, NL_THREADS, 0, st>>>(a, rec);
+    k_near_leaf<true, true><<<ntask, NL_THREADS, 0, st>>>(a, tasks);
   else if (a.dosl)
-    k_near_leaf<true, false><<<grid, NL_THREADS, 0, st>>>(a, rec);
+    k_near_leaf<true, false><<<ntask, NL_THREADS, 0, st>>>(a, tasks);
   else
-    k_near_leaf<false, true><<<grid, NL_THREADS, 0, st>>>(a, rec);
+    k_near_leaf<false, true><<<ntask, NL_THREADS, 0, st>>>(a, tasks);
   count_launch();
 }
 
 void launch_near_store(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
-                       int dodisp, double* store) {
+                       double* store) {
   if (a.nleaf <= 0) return;
-  k_near_store<<<a.nleaf, NF_WARPS * 32, 0, st>>>(a, base, ntri, K, dodisp, store); count_launch();
+  k_near_store<<<dim3(a.nleaf, 16), NF_WARPS * 32, 0, st>>>(a, base, ntri, K, store); count_launch();
 }
 
 void launch_near_replay(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
@@ -927,52 +874,53 @@ void launch_near_replay(cudaStream_t st, const NearArgs& a, const long long* bas
   k_near_replay<<<a.nleaf, 256, 0, st>>>(a, base, ntri, K, dodisp, ssl, sdl, store); count_launch();
 }
 
-void launch_near_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int* chunk_leaf,
-                       const int* chunk_e0, int R, int dostrain, const double* ssl, const double* sdl,
-                       int ntri_all, int nsrc, int ntgt, const long long* sbase, const int* sntri,
-                       const double* store) {
-  if (nchunk <= 0 || R <= 0) return;
+void launch_near_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R, int dostrain,
+                       const double* ssl, const double* sdl, int nsrc, int ntgt) {
+  if (ntask <= 0 || R <= 0) return;
   if (R > 64) throw CudaError{(int)cudaErrorInvalidValue};
-  const int nl = a.dosl + a.dodl;
-  const int K = nl * 3 * (3 + 6 * dostrain);
+  const int K = (a.dosl + a.dodl) * 3 * (3 + 6 * dostrain);
   const int RB = (R + 15) / 16;
   const int smem = (int)(sizeof(double) * (NB_PTS * NB_TRI * K + NB_TRI * 6 * 16 * RB));
   auto go = [&](auto kern) {
     EFMM_CUDA_TRY(smem_raise(kern, (int)(smem)));
-    kern<<<nchunk, NB_THREADS, smem, st>>>(a, chunk_leaf, chunk_e0, R, K, dostrain, ssl, sdl, ntri_all, nsrc,
-                                           ntgt, sbase, sntri, store);
+    kern<<<ntask, NB_THREADS, smem, st>>>(a, tasks, R, K, dostrain, ssl, sdl, nsrc, ntgt);
     count_launch();
   };
-  if (store) {
-    const int nlay = nl, str = dostrain;
-    const double* g0 = a.dosl ? ssl : sdl;
-    const double* g1 = sdl;
-    const int smem2 = (int)(sizeof(double) * (NB_PTS * NB_TRI * K + NB_TRI * 3 * nlay * 16 * RB));
-    auto go2 = [&](auto kern) {
-      EFMM_CUDA_TRY(smem_raise(kern, (int)(smem2)));
-      kern<<<nchunk, NB_THREADS, smem2, st>>>(a, chunk_leaf, chunk_e0, R, g0, g1, nsrc, ntgt, sbase, sntri, store);
-      count_launch();
-    };
-#define EFMM_RB(RBV)                                                         \
-  if (nlay == 1 && !str) go2(k_near_replay_batch<RBV, 1, 0>);                \
-  else if (nlay == 1) go2(k_near_replay_batch<RBV, 1, 1>);                   \
-  else if (!str) go2(k_near_replay_batch<RBV, 2, 0>);                        \
-  else go2(k_near_replay_batch<RBV, 2, 1>);
-    switch (RB) {
-      case 1: EFMM_RB(1) break;
-      case 2: EFMM_RB(2) break;
-      case 3: EFMM_RB(3) break;
-      default: EFMM_RB(4) break;
-    }
-#undef EFMM_RB
-  } else {
-    switch (RB) {
-      case 1: go(k_near_batch<1, false>); break;
-      case 2: go(k_near_batch<2, false>); break;
-      case 3: go(k_near_batch<3, false>); break;
-      default: go(k_near_batch<4, false>); break;
-    }
+  switch (RB) {
+    case 1: go(k_near_batch<1>); break;
+    case 2: go(k_near_batch<2>); break;
+    case 3: go(k_near_batch<3>); break;
+    default: go(k_near_batch<4>); break;
   }
+  EFMM_CUDA_TRY(cudaGetLastError());
+}
+
+void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int* chunk_leaf,
+                              const int* chunk_e0, int R, int dostrain, const double* ssl, const double* sdl,
+                              int nsrc, int ntgt, const long long* sbase, const int* sntri, const double* store) {
+  if (nchunk <= 0 || R <= 0) return;
+  if (R > 64) throw CudaError{(int)cudaErrorInvalidValue};
+  const int nlay = a.dosl + a.dodl, str = dostrain, K = nlay * 3 * (3 + 6 * dostrain), RB = (R + 15) / 16;
+  const double* g0 = a.dosl ? ssl : sdl;
+  const double* g1 = sdl;
+  const int smem = (int)(sizeof(double) * (NB_PTS * NB_TRI * K + NB_TRI * 3 * nlay * 16 * RB));
+  auto go = [&](auto kern) {
+    EFMM_CUDA_TRY(smem_raise(kern, (int)(smem)));
+    kern<<<nchunk, NB_THREADS, smem, st>>>(a, chunk_leaf, chunk_e0, R, g0, g1, nsrc, ntgt, sbase, sntri, store);
+    count_launch();
+  };
+#define EFMM_RB(RBV)                                                        \
+  if (nlay == 1 && !str) go(k_near_replay_batch<RBV, 1, 0>);                \
+  else if (nlay == 1) go(k_near_replay_batch<RBV, 1, 1>);                   \
+  else if (!str) go(k_near_replay_batch<RBV, 2, 0>);                        \
+  else go(k_near_replay_batch<RBV, 2, 1>);
+  switch (RB) {
+    case 1: EFMM_RB(1) break;
+    case 2: EFMM_RB(2) break;
+    case 3: EFMM_RB(3) break;
+    default: EFMM_RB(4) break;
+  }
+#undef EFMM_RB
   EFMM_CUDA_TRY(cudaGetLastError());
 }
 
@@ -989,8 +937,10 @@ void launch_direct_all(cudaStream_t st, int ntri, const TriEdge* rec, int nsrc, 
     EFMM_CUDA_TRY(cudaMemsetAsync(u_tgt, 0, 24 * (size_t)ntgt, st));
     EFMM_CUDA_TRY(cudaMemsetAsync(e_tgt, 0, 48 * (size_t)ntgt, st));
   }
-  const int nb = (nep + NL_THREADS - 1) / NL_THREADS;
-  const dim3 grid(nb, near_split(nb, ntri));
+  // parts of the triangles so that few points still cover the chip about
+  // three times (3 CTAs per SM), but no part of fewer than about 16
+  const int nb = (nep + NL_THREADS - 1) / NL_THREADS, want = (3 * 3 * 148 + nb - 1) / nb;
+  const dim3 grid(nb, std::max(1, std::min({want, (ntri + 15) / 16, 64})));
   auto go = [&](auto kern) {
     kern<<<grid, NL_THREADS, 0, st>>>(ntri, rec, nsrc, src_pts, ntgt, tgt_pts, dostrain_src, dostrain_tgt, rlam, rmu,
                                       u_src, e_src, u_tgt, e_tgt);

@@ -108,7 +108,7 @@ extern "C" int efmm_direct_noalloc(double rlam, double rmu, int n, const double*
   int do_src = (u_src || e_src) ? n : 0;
   int do_tgt = (nt > 0 && (u_tgt || e_tgt)) ? nt : 0;
   try {
-    launch_tri_edge_prep(st, n, tri, nullptr, ssl, sdl, dosl, dodl, S.tri);
+    launch_tri_edge_prep(st, n, tri, ssl, sdl, dosl, dodl, S.tri);
     launch_direct_all(st, n, S.tri, do_src, src, do_tgt, tgt, dosl, dodl, e_src ? 1 : 0,
                       e_tgt ? 1 : 0, rlam, rmu, S.u, S.e, S.u + 3 * (size_t)n, S.e + 6 * (size_t)n);
     if (do_src) {

@@ -265,6 +265,7 @@ class Plan {
   void ensure_mats_f();
   int build_image_sched();
   void build_chunks(int do_src, int do_tgt);
+  void build_near_tasks(int do_src, int do_tgt, int pts);
   bool mindlin_ = false, img_sched_ = false;
   bool forest_on_ = false;
   // keep the geometry-only features of the two-stage P2M / L2T between
@@ -311,6 +312,8 @@ class Plan {
   DevBuf<float> mpole_f_, local_f_;
   DevBuf<int> chunk_leaf_, chunk_e0_;  // (near leaf, first point) per batched near-field CTA
   int nchunk_ = 0, chunk_key_ = -1;
+  DevBuf<NearTask> ntask_;  // work items of the one-right-hand-side near field
+  int nntask_ = 0, ntask_key_ = -1;
   std::vector<int> l2t_sc_h_, l2t_tc_h_;  // per L2T leaf
   std::vector<int> l2t_h_;                // L2T leaves
   DevBuf<double> l2t_scratch_;            // functionals + sums of one wave of leaves
@@ -349,6 +352,10 @@ class Plan {
   int np2m_ = 0, nl2t_ = 0, nnear_ = 0;
   std::vector<int> near_sc_h_, near_tc_h_, near_ntri_h_;  // per near leaf
   DevBuf<int> near_ntri_;
+  DevBuf<int> near_rstart_;  // near triangles as ranges (NearArgs::rng)
+  DevBuf<int2> near_rng_;
+  std::vector<int> near_rstart_h_;
+  std::vector<int2> near_rng_h_;
   DevBuf<long long> near_base_;
   std::vector<long long> near_base_h_;
   // FP32 product-layout copy of the stored near field for mixed replays on
@@ -429,7 +436,6 @@ class Plan {
   DevBuf<int> m2l_cnt_, m2l_cursor_;
   DevBuf<double> mpole_, local_;
   DevBuf<double> ssl_s_, sdl_s_, u_s_, e_s_, ut_s_, et_s_;
-  DevBuf<TriRec> trir_;
   DevBuf<TriEdge> tedge_;
   OpPool* ops_ = nullptr;
   cudaEvent_t ev_[10];

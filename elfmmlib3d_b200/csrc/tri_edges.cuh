@@ -21,9 +21,14 @@
 // terms on either side of the foot of the target (rho = 0 included: targets
 // collinear with an edge), one division and one logarithm per edge.
 //
-// Compared with the derivative tables of tri_integrals.cuh (45 entries per
-// pair, rotated per edge, then contracted): about half the FP64 operations
-// and half the registers.
+// Compared with derivative tables of the integrals of r and 1/r in the
+// triangle frame (45 entries per pair, as the reference's triartable and
+// triabtable, src/triahquad.f:680 and :797, rotated per edge, then contracted,
+// the form used before): about half the FP64 operations and two thirds of the
+// registers, errors against long double equal to within 1.3x from 1 to 30
+// edge lengths.  On-surface evaluation (target on its own triangle) uses h =
+// 0, Omega = 0: the principal value / Hadamard finite part, the reference's
+// iquad = 0 convention (src/triahquad.f:4037-4055).
 #pragma once
 #include "tri_index.cuh"
 
@@ -232,6 +237,170 @@ EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool st
       for (int c = 0; c < 3; c++) y[c] = f * (Mn[c] + nn * n[c]) - 2.0 * i2mu * om * s[c];
       te_sym(e, 1.0, n, y);
     }
+  }
+}
+
+// The quantities of edge k of T that both layers' unit responses use.
+struct TeEdge {
+  double t[3], nu[3], rho[3], v, h, RA, RB, uA, uB, iA, iB, L, K3, K5;
+};
+EFMM_HD bool te_edge(const TriEdge& T, int k, const double r[3][3], const double R[3], const double iR[3], double h,
+                     TeEdge& g) {
+  double rA[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    rA[c] = k == 0 ? r[0][c] : (k == 1 ? r[1][c] : r[2][c]);
+    g.t[c] = T.t[3 * k + c];
+  }
+  g.RA = k == 0 ? R[0] : (k == 1 ? R[1] : R[2]);
+  g.RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
+  g.iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
+  g.iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
+  g.uA = te_dot(rA, g.t);
+  g.uB = g.uA - T.len[k];
+  te_cross(g.t, T.n, g.nu);
+  g.v = te_dot(rA, g.nu);
+  g.h = h;
+#pragma unroll
+  for (int c = 0; c < 3; c++) g.rho[c] = g.v * g.nu[c] + h * T.n[c];
+  return te_line(T.len[k], g.uA, g.uB, g.RA, g.RB, g.iA, g.iB, g.v * g.v + h * h, g.L, g.K3, g.K5);
+}
+// e += f sym(e_k, b)
+EFMM_HD void te_sym_axis(double* e, int k, double f, const double* b) {
+  const double h = 0.5 * f;
+  if (k == 0) {
+    e[0] += f * b[0]; e[3] += h * b[1]; e[4] += h * b[2];
+  } else if (k == 1) {
+    e[1] += f * b[1]; e[3] += h * b[0]; e[5] += h * b[2];
+  } else {
+    e[2] += f * b[2]; e[4] += h * b[0]; e[5] += h * b[1];
+  }
+}
+
+// Unit responses of one (triangle, target) pair, the stored near-field
+// operator of the ITER mode (src/elfmm3dtria_iter_1.f:1559-1760 stores the
+// same three unit responses): LAYER 0 single, 1 double; out[KB k + (0..2 u,
+// 3..8 strain)] for a unit density along each axis k, KB = 9 with strain, else
+// 3.  The arithmetic of tri_edge_pair with the tensors that do not depend on
+// the density formed once per edge.
+template <int LAYER, bool STR>
+EFMM_HD void tri_edge_blocks(const TriEdge& T, const double* X, bool self, double al, double i2mu, double* out) {
+  constexpr int KB = STR ? 9 : 3;
+  double r[3][3], R[3], iR[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[k][c] = X[c] - T.v[3 * k + c];
+    R[k] = sqrt(te_dot(r[k], r[k]));
+    iR[k] = 1.0 / R[k];
+  }
+  const double h = self ? 0.0 : te_dot(r[0], T.n);
+  double om = 0.0;
+  if (h != 0.0) {
+    const double den = R[0] * R[1] * R[2] + te_dot(r[0], r[1]) * R[2] + te_dot(r[0], r[2]) * R[1] +
+                       te_dot(r[1], r[2]) * R[0];
+    om = 2.0 * atan2(h * T.area2, den);
+  }
+  double o[27];
+#pragma unroll
+  for (int q = 0; q < 27; q++) o[q] = 0.0;
+  double N = 0.0, kz = 0.0, unn[3] = {0, 0, 0}, knn[3] = {0, 0, 0};
+#pragma unroll 1
+  for (int k = 0; k < 3; k++) {
+    TeEdge g;
+    if (!te_edge(T, k, r, R, iR, h, g)) continue;
+    const double di = g.iA - g.iB;
+    if (LAYER == 1) {
+      const double* t = g.t;
+      const double d3 = g.iA * g.iA * g.iA - g.iB * g.iB * g.iB;
+      const double du3 = g.uA * g.iA * g.iA * g.iA - g.uB * g.iB * g.iB * g.iB;
+      double c[3], q[3];
+      te_cross(t, g.rho, c);
+#pragma unroll
+      for (int j = 0; j < 3; j++) q[j] = g.K3 * g.rho[j] - di * t[j];
+      double A[6] = {0, 0, 0, 0, 0, 0}, gx[3];
+      if (STR) {
+        const double m[3] = {2.0 * d3 * t[0] - 3.0 * g.K5 * g.rho[0], 2.0 * d3 * t[1] - 3.0 * g.K5 * g.rho[1],
+                             2.0 * d3 * t[2] - 3.0 * g.K5 * g.rho[2]};
+        te_sym(A, al, g.rho, m);
+        te_sym(A, al * (du3 - g.K3), t, t);
+        A[0] += al * g.K3;
+        A[1] += al * g.K3;
+        A[2] += al * g.K3;
+#pragma unroll
+        for (int j = 0; j < 3; j++) gx[j] = g.K3 * (g.v * T.n[j] - h * g.nu[j]);
+      }
+      const double fw = (1.0 - al) * g.L;
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        double* u = o + 9 * j;
+        double* e = u + 3;
+        const int j1 = j == 2 ? 0 : j + 1, j2 = j == 0 ? 2 : j - 1;
+        // w = e_j x t: component j1 -t[j2], component j2 t[j1]
+        const double s = al * c[j];
+        u[0] += s * q[0];
+        u[1] += s * q[1];
+        u[2] += s * q[2];
+        u[j1] -= fw * t[j2];
+        u[j2] += fw * t[j1];
+        if (STR) {
+#pragma unroll
+          for (int z = 0; z < 6; z++) e[z] += c[j] * A[z];
+          te_sym_axis(e, j1, -(2.0 * al - 1.0) * t[j2], q);
+          te_sym_axis(e, j2, (2.0 * al - 1.0) * t[j1], q);
+          te_sym_axis(e, j, 1.0, gx);
+        }
+      }
+    } else {
+      const double Et = T.len[k] * (g.uA + g.uB) / (g.RA + g.RB), hL = h * g.L;
+      const double du = g.uA * g.iA - g.uB * g.iB, kn = g.L - h * h * g.K3;
+      N -= g.v * g.L;
+      double B[6] = {0, 0, 0, 0, 0, 0}, Tn[6] = {0, 0, 0, 0, 0, 0}, Rn[6] = {0, 0, 0, 0, 0, 0};
+      if (STR) {
+        kz -= g.v * h * g.K3;
+        te_sym(B, i2mu * al, g.nu, T.n);   // in-plane rows' normal column
+        te_sym(Tn, i2mu * al, g.nu, g.t);
+        te_sym(Rn, i2mu * al, g.nu, g.rho);
+      }
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        double* u = o + 9 * j;
+        double* e = u + 3;
+        const double st = g.t[j], sr = g.rho[j];
+        const double f = i2mu * al * (st * Et + sr * g.L);
+#pragma unroll
+        for (int z = 0; z < 3; z++) u[z] += f * g.nu[z];
+        unn[j] += g.nu[j] * hL;
+        if (STR) {
+          const double ct = st * (du - g.L) + sr * di, cr = st * di - g.K3 * sr;
+          const double gn = cr * h + g.L * T.n[j];
+#pragma unroll
+          for (int z = 0; z < 6; z++) e[z] += ct * Tn[z] + cr * Rn[z] + gn * B[z];
+          te_sym_axis(e, j, i2mu * (al - 2.0) * g.L, g.nu);
+          knn[j] -= g.nu[j] * kn;
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    double* u = o + 9 * j;
+    double* e = u + 3;
+    if (LAYER == 1) {
+      u[j] += om;
+    } else {
+      const double Nh = N - h * om, sn = T.n[j];
+      const double fn = i2mu * al * (unn[j] - sn * (2.0 * Nh - N));
+#pragma unroll
+      for (int z = 0; z < 3; z++) u[z] += fn * T.n[z];
+      u[j] += i2mu * 2.0 * Nh;
+      if (STR) {
+        te_sym(e, -i2mu * al * (knn[j] + sn * (kz - 2.0 * om)), T.n, T.n);
+        te_sym_axis(e, j, -2.0 * i2mu * om, T.n);
+      }
+    }
+#pragma unroll
+    for (int z = 0; z < KB; z++) out[KB * j + z] = u[z];
   }
 }
 

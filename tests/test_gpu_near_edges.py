@@ -59,3 +59,30 @@ def test_split_leaves_match_direct(gpu, level, iprec):
     ud, ed, _, _ = gpu.el3dtriadirecttarg(1.0, 1.0, tri, nrm, cen, ssl, sdl)
     tol = {1: 5e-4, 2: 5e-6}[iprec]
     assert rel(u, ud) < tol and rel(e, ed) < 10 * tol
+
+
+@pytest.mark.parametrize("nrhs", [1, 4, 5, 16, 17])
+@pytest.mark.parametrize("n,m", [(7, 0), (33, 9), (130, 50)])
+@pytest.mark.parametrize("sl,dl,strain", [(True, True, True), (False, True, True), (True, False, False)])
+def test_batch_equals_single_calls(gpu, nrhs, n, m, sl, dl, strain):
+    """Both sides of the rule that runs few right-hand sides one by one."""
+    import torch
+    tri, nrm, cen = _soup(n, n + 1)
+    rng = np.random.default_rng(3)
+    d = lambda a: torch.tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")
+    z = lambda *s: torch.zeros(s, dtype=torch.float64, device="cuda")
+    P = gpu.Plan(0)
+    P.set_geometry(d(tri), d(nrm), d(cen), d(rng.uniform(-5, 5, (m, 3))) if m else None, iprec=5)
+    ssl, sdl = (d(rng.normal(size=(nrhs, n, 3))) if on else None for on in (sl, dl))
+    mk = lambda *lead: [z(*lead, n, 3), z(*lead, n, 3, 3) if strain else None, z(*lead, m, 3) if m else None,
+                        z(*lead, m, 3, 3) if m and strain else None]
+    batch = mk(nrhs)
+    P.evaluate_batch(1.3, 0.7, nrhs, ssl, sdl, *batch)
+    for r in range(nrhs):
+        one = mk()
+        P.evaluate(1.3, 0.7, None if ssl is None else ssl[r], None if sdl is None else sdl[r], *one)
+        for a, b in zip(batch, one):
+            if a is not None:
+                # the same closed forms; cancellation inside a pair's response up to about 1e4
+                assert rel(a[r].cpu().numpy(), b.cpu().numpy()) < 1e-11
+    P.close()
