@@ -717,17 +717,76 @@ void Plan::ensure_factored(bool tc) {
     if (P->rot_ready) return;
   }
   // device layout: blocks column-major
-  column_major_factored(rops, pool);
   {
     std::vector<double> tmp(poolf.begin(), poolf.end());
     column_major_factored(rops, tmp);
     for (size_t i = 0; i < tmp.size(); i++) poolf[i] = (float)tmp[i];
   }
   h2d(P->rot_ops, rops, st_);
-  h2d(P->rot_d, pool, st_);
   h2d(P->rot_f, poolf, st_);
   EFMM_CUDA_TRY(cudaStreamSynchronize(st_));
   P->rot_ready = true;
+}
+
+// FP64 tensor-core translations: one launch per level and tile width, the
+// largest orders first.
+void Plan::cut_mma_tasks(TransSched& S, int C) {
+  if (S.mC == C && S.mpool == ops_) return;
+  std::vector<TransTask> tasks;
+  S.mb.clear();
+  for (auto& r : S.lev) {
+    if (r.second == 0) continue;
+    std::vector<int> segs(r.second);
+    double cols = 0;
+    for (int q = 0; q < r.second; q++) {
+      segs[q] = r.first + q;
+      cols += (double)S.segs[segs[q]].npair * C / r.second;
+    }
+    const std::vector<OpDesc>& od = ops_->descs;
+    std::stable_sort(segs.begin(), segs.end(),
+                     [&](int a, int b) { return od[S.segs[a].group].p > od[S.segs[b].group].p; });
+    for (size_t i = 0; i < segs.size();) {
+      const int pmax = od[S.segs[segs[i]].group].p, nt = rot_mma_tiles(pmax, cols), t0 = (int)tasks.size();
+      const bool big = rot_mma_big(pmax, nt);
+      for (; i < segs.size(); i++) {
+        const TransSeg& g = S.segs[segs[i]];
+        const int pg = od[g.group].p;
+        if (rot_mma_tiles(pg, cols) != nt || rot_mma_big(pg, nt) != big) break;
+        const int ncols = g.npair * C;
+        for (int c0 = 0; c0 < ncols; c0 += 8 * nt) tasks.push_back({g.group, 0, g.pair0, ncols, c0});
+      }
+      S.mb.push_back({t0, (int)tasks.size() - t0, pmax, nt});
+    }
+  }
+  h2d(S.mtasks, tasks, st_);
+  S.mC = C;
+  S.mpool = ops_;
+}
+
+// FP64 operators of the pool (rotations.cu build_mma_ops), once per pool
+void Plan::ensure_mma() {
+  std::lock_guard<std::mutex> lk(g_ops_mu);
+  OpPool* P = ops_;
+  if (P->rotm_ready) return;
+  std::vector<int> kinds, orders;
+  std::vector<double> offs;
+  for (const OpDesc& d : P->descs) {
+    kinds.push_back(d.kind);
+    orders.push_back(d.p);
+    offs.insert(offs.end(), {d.d[0], d.d[1], d.d[2]});
+  }
+  std::vector<RotMOp> mops;
+  std::vector<double> pool;
+  std::vector<unsigned char> s16, s8;
+  build_mma_ops(kinds, orders, offs, mops, pool);
+  build_rm_sched(16, s16);
+  build_rm_sched(8, s8);
+  h2d(P->rotm_ops, mops, st_);
+  h2d(P->rotm_d, pool, st_);
+  h2d(P->rotm_s16, s16, st_);
+  h2d(P->rotm_s8, s8, st_);
+  EFMM_CUDA_TRY(cudaStreamSynchronize(st_));
+  P->rotm_ready = true;
 }
 
 // parity-split FP32 operators (rotations.cu build_split_ops), once per pool
@@ -926,32 +985,40 @@ void Plan::run_translations(TransSched& S, int C, const T* mats, const T* src, T
       return;
     }
   }
-  // factored form when its column tiles fit in shared memory
-  // (the split kernel's tiles have rot_split_cols() columns; the split
-  // serves every launch when it is on: p <= 31 bounds every group's order)
-  const bool split = sizeof(T) == 4 && split_rot();
-  const int W = split ? rot_split_cols() : rot_cols_per_cta(D, (int)sizeof(T));
-  const size_t smem = sizeof(T) * 2 * (size_t)D * rot_cols_per_cta(D, (int)sizeof(T));
-  if (factored_ && smem <= 227 * 1024) {
-    ensure_factored();
-    cut_rot_tasks(S, C, W);
-    const T* pool = nullptr;
-    if (sizeof(T) == 8)
-      pool = reinterpret_cast<const T*>(ops_->rot_d.get());
-    else
-      pool = reinterpret_cast<const T*>(ops_->rot_f.get());
-    if (split) ensure_split();
-    for (size_t i = 0; i < S.lev_rtasks.size(); i++) {
-      if (split && rot_split_ok(S.lev_rdim[i])) {
-        launch_translate_rot_split(st_, S.lev_rtasks[i].second, S.rtasks.get() + S.lev_rtasks[i].first,
-                                   S.pairs.get(), ops_->rots_ops.get(), ops_->rots_f.get(), D, C, S.lev_rdim[i],
-                                   reinterpret_cast<const float*>(src), reinterpret_cast<float*>(dst));
-        continue;
-      }
-      launch_translate_rot<T>(st_, S.lev_rtasks[i].second, S.rtasks.get() + S.lev_rtasks[i].first, S.pairs.get(),
-                              ops_->rot_ops.get(), pool, D, C, S.lev_rdim[i], src, dst);
+  if constexpr (sizeof(T) == 8) {
+    // factored form on the FP64 tensor cores when its rows fit in shared memory
+    if (factored_ && rot_mma_ok(p_)) {
+      ensure_mma();
+      cut_mma_tasks(S, C);
+      for (const TransSched::MmaBatch& b : S.mb)
+        launch_translate_mma(st_, b.ntask, S.mtasks.get() + b.task0, S.pairs.get(), ops_->rotm_ops.get(),
+                             ops_->rotm_d.get(), ops_->rotm_s16.get(), ops_->rotm_s8.get(), D, C, b.pmax, b.nt, src,
+                             dst);
+      return;
     }
-    return;
+  } else {
+    // factored form when its column tiles fit in shared memory
+    // (the split kernel's tiles have rot_split_cols() columns; the split
+    // serves every launch when it is on: p <= 31 bounds every group's order)
+    const bool split = split_rot();
+    const int W = split ? rot_split_cols() : rot_cols_per_cta(D, (int)sizeof(T));
+    const size_t smem = sizeof(T) * 2 * (size_t)D * rot_cols_per_cta(D, (int)sizeof(T));
+    if (factored_ && smem <= 227 * 1024) {
+      ensure_factored();
+      cut_rot_tasks(S, C, W);
+      if (split) ensure_split();
+      for (size_t i = 0; i < S.lev_rtasks.size(); i++) {
+        if (split && rot_split_ok(S.lev_rdim[i])) {
+          launch_translate_rot_split(st_, S.lev_rtasks[i].second, S.rtasks.get() + S.lev_rtasks[i].first,
+                                     S.pairs.get(), ops_->rots_ops.get(), ops_->rots_f.get(), D, C, S.lev_rdim[i],
+                                     src, dst);
+          continue;
+        }
+        launch_translate_rot<T>(st_, S.lev_rtasks[i].second, S.rtasks.get() + S.lev_rtasks[i].first, S.pairs.get(),
+                                ops_->rot_ops.get(), ops_->rot_f.get(), D, C, S.lev_rdim[i], src, dst);
+      }
+      return;
+    }
   }
   cut_tasks(S, C);
   for (auto& r : S.lev_tasks)

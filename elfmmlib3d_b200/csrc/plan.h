@@ -31,11 +31,16 @@ struct OpPool {
   std::vector<OpDesc> descs;
   DevBuf<int> m2lg_dev;  // m2l_group on the device
   // factored form (rotation, shift along z, rotation back) of every group,
-  // FP64 factorial basis and FP32 normalised basis; made on first use
+  // FP32 normalised basis; made on first use
   bool rot_ready = false;
   DevBuf<RotOp> rot_ops;
-  DevBuf<double> rot_d;
   DevBuf<float> rot_f;
+  // the FP64 operators in the parity-split form for the FP64 tensor cores
+  // and the block lists of 16 and 8 warps; made on the first FP64 pass
+  bool rotm_ready = false;
+  DevBuf<RotMOp> rotm_ops;
+  DevBuf<double> rotm_d;
+  DevBuf<unsigned char> rotm_s16, rotm_s8;
   // the FP32 factored operators as tensor-core tiles (orders <= 31); made on
   // the first FP32 pass that uses them
   bool rot_tc_ready = false;
@@ -94,6 +99,15 @@ struct TransSched {
   DevBuf<TransTask> rtasks;
   std::vector<std::pair<int, int>> lev_rtasks;  // task ranges in execution order,
   std::vector<int> lev_rdim;                     // each with its largest operator size
+  // FP64 tensor-core form: column tiles of 8 nt columns, per launch their
+  // range, the largest order and nt
+  int mC = -1;
+  const void* mpool = nullptr;
+  DevBuf<TransTask> mtasks;
+  struct MmaBatch {
+    int task0, ntask, pmax, nt;
+  };
+  std::vector<MmaBatch> mb;
   // tensor-core form: segments, 32-column tasks, and per launch (a level,
   // or all levels of an M2L stage) the task range and its largest order
   int tcC = -1;
@@ -112,7 +126,7 @@ struct TransSched {
     segs.clear();
     lev.clear();
     C = -1;
-    pool = rpool = nullptr;
+    pool = rpool = mpool = nullptr;
     lev_tasks.clear();
     rC = rW = -1;
     lev_rtasks.clear();
@@ -396,6 +410,8 @@ class Plan {
   void cut_tasks(TransSched& S, int C, const std::vector<int>* dims = nullptr);
   void cut_rot_tasks(TransSched& S, int C, int W);
   void ensure_factored(bool tc = false);
+  void cut_mma_tasks(TransSched& S, int C);
+  void ensure_mma();
   void ensure_split();
   // the U-kernel M2L in the parity-split form (mixed form; ELFMM3D_USPLIT=0:
   // the dense FP32 operators)

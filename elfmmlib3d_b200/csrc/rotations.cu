@@ -619,6 +619,46 @@ void build_split_ops(const std::vector<int>& kinds, const std::vector<int>& orde
   });
 }
 
+void build_mma_ops(const std::vector<int>& kinds, const std::vector<int>& orders, const std::vector<double>& offsets,
+                   std::vector<RotMOp>& ops, std::vector<double>& pool) {
+  const int ng = (int)kinds.size();
+  int pmax = 0;
+  for (int q : orders) pmax = std::max(pmax, q);
+  Fitter F;
+  F.init(pmax);
+  ops.resize(ng);
+  long long off = 0;
+  for (int g = 0; g < ng; g++) {
+    ops[g] = {orders[g], 0, off};
+    off += rm_group_size(orders[g]);
+  }
+  pool.assign((size_t)off, 0.0);
+  parallel_for(ng, [&](int g) {
+    const int p = orders[g];
+    SplitHost S;
+    build_split_host(kinds[g], p, &offsets[3 * g], F, S);
+    double* o = &pool[ops[g].base];
+    std::copy(S.rz[0].begin(), S.rz[0].begin() + 4 * (p + 1), o);
+    std::copy(S.rz[1].begin(), S.rz[1].begin() + 4 * (p + 1), o + 4 * (p + 1) + 3 * rm_stage_size(p));
+    // block of r rows, rows and columns from i0 of a full block of rf rows
+    auto pack = [&](int stage, const std::vector<double>& B, int rf, int part, int i0) {
+      const int r = rf - i0, mt = (r + 7) / 8;
+      if (r <= 0) return;
+      double* d = o + 4 * (p + 1) + stage * rm_stage_size(p) + rm_block_off(p, r, part);
+      for (int i = 0; i < r; i++)
+        for (int k = 0; k < r; k++)
+          d[((k / 4) * mt + i / 8) * 32 + (i % 8) * 4 + k % 4] = B[(size_t)part * rf * rf + (size_t)(i + i0) * rf + k + i0];
+    };
+    for (int n = 0; n <= p; n++)
+      for (int part = 0; part < 2; part++) {
+        pack(0, S.ry[0][n], n + 1, part, part);  // the im part has no order 0
+        pack(2, S.ry[1][n], n + 1, part, part);
+      }
+    for (int m = 0; m <= p; m++)
+      for (int part = 0; part < (m > 0 ? 2 : 1); part++) pack(1, S.z[m], p - m + 1, part, 0);
+  });
+}
+
 // ------------------------------ M2L of the half-space kernel U, parity split
 // U is unchanged by rotations about z and by the reflection y -> -y, so its
 // M2L operator for an offset d = (rho cos phi, rho sin phi, dz) is
@@ -1576,8 +1616,6 @@ void launch_translate_rot(cudaStream_t st, int ntask, const TransTask* tasks, co
   kern<<<ntask, ROT_THREADS, smem, st>>>(tasks, pairs, ops, pool, D, C, src, dst); count_launch();
   EFMM_CUDA_TRY(cudaGetLastError());
 }
-template void launch_translate_rot<double>(cudaStream_t, int, const TransTask*, const TransPair*, const RotOp*,
-                                           const double*, int, int, int, const double*, double*);
 template void launch_translate_rot<float>(cudaStream_t, int, const TransTask*, const TransPair*, const RotOp*,
                                           const float*, int, int, int, const float*, float*);
 

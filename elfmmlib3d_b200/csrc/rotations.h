@@ -68,6 +68,25 @@ void build_split_ops(const std::vector<int>& kinds, const std::vector<int>& orde
 // Whether the split kernel serves a launch whose largest operator size is maxdim.
 bool rot_split_ok(int maxdim);
 
+// The parity-split form in FP64 (factorial basis) for the FP64 tensor cores
+// (rot_mma.cu): per group Rz, the re / im blocks of Ry, of the shift and of
+// Ry back in mma fragment order, Rz back, at base (doubles).
+struct RotMOp {
+  int p, pad;
+  long long base;
+};
+constexpr int RM_PMAX = 41;   // largest order: 16 columns of (p + 1)^2 rows fit in shared memory
+constexpr int RM_UNITS = 64;  // bytes of a warp's block list
+long long rm_group_size(int p);
+long long rm_stage_size(int p);
+long long rm_block_off(int p, int r, int part);
+void build_rm_sched(int nw, std::vector<unsigned char>& out);
+void build_mma_ops(const std::vector<int>& kinds, const std::vector<int>& orders, const std::vector<double>& offsets,
+                   std::vector<RotMOp>& ops, std::vector<double>& pool);
+bool rot_mma_ok(int p);
+int rot_mma_tiles(int p, double cols);
+bool rot_mma_big(int p, int nt);  // a launch of 16-warp CTAs, one per SM
+
 // M2L of the half-space kernel U in the parity-split form (FP32 normalised
 // pool): per group the order, the leading dimension of its blocks (ncoef
 // rounded up to 4), the offsets (floats) of its re and im blocks (row-major,
@@ -85,6 +104,13 @@ void build_usplit_ops(const std::vector<int>& orders, const std::vector<double>&
 
 struct TransTask;
 struct TransPair;
+
+// FP64: apply the translations of ntask tiles of 8 nt columns (task.col0
+// counts columns of the group's pairs x C), orders <= pmax, and ADD into dst.
+void launch_translate_mma(cudaStream_t st, int ntask, const TransTask* tasks, const TransPair* pairs,
+                          const RotMOp* ops, const double* pool, const unsigned char* sched16,
+                          const unsigned char* sched8, int D, int C, int pmax, int nt, const double* src,
+                          double* dst);
 
 // Apply the factored translations of ntask column tiles (task.col0 counts
 // columns of the group's pairs x C; task.row0 unused) and ADD into dst.
