@@ -6,12 +6,12 @@
 
 namespace efmm {
 
-// Work item of the one-right-hand-side near field: evaluation points
+// Work item of the near field: evaluation points
 // [e0, e0 + ne) of near leaf li against cnt triangles of its list from
-// offset k0 of its range r0; shared: other items hold more of the leaf's
-// triangles for the same points (outputs added atomically).
+// position p0 (offset k0 of its range r0); shared: other items hold more of
+// the leaf's triangles for the same points (outputs added atomically).
 struct NearTask {
-  int li, e0, ne, r0, k0, cnt, shared;
+  int li, e0, ne, r0, k0, p0, cnt, shared;
 };
 
 struct NearArgs {
@@ -39,18 +39,16 @@ void launch_near_leaf(cudaStream_t st, const NearArgs& a, int ntask, const NearT
 constexpr int NEAR_TASK_PTS = 128;  // evaluation points of a work item, at most
 void launch_near_store(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
                        double* store);
-void launch_near_replay(cudaStream_t st, const NearArgs& a, const long long* base, const int* ntri, int K,
-                        int dodisp, const double* ssl, const double* sdl, const double* store);
 // R <= 64 right-hand sides; densities (n, 3, R) tree order, outputs (R, nsrc
 // or ntgt, 3 or 6) tree order, ADDED to.  Items of at most NEAR_BATCH_PTS points.
 constexpr int NEAR_BATCH_PTS = 8;
 void launch_near_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R, int dostrain,
                        const double* ssl, const double* sdl, int nsrc, int ntgt);
 // The same with the pair blocks of the ITER store (per leaf at sbase, sntri
-// near triangles), over chunks of 8 evaluation points.
-void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int nchunk, const int* chunk_leaf,
-                              const int* chunk_e0, int R, int dostrain, const double* ssl, const double* sdl,
-                              int nsrc, int ntgt, const long long* sbase, const int* sntri, const double* store);
+// near triangles).
+void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R,
+                              int dostrain, const double* ssl, const double* sdl, int nsrc, int ntgt,
+                              const long long* sbase, const int* sntri, const double* store);
 // Mixed-precision replay of the stored near field on the tensor cores: the
 // FP64 store converted once to FP32 in the product layout (per leaf at the
 // store's offsets: A[NJ t + j][KB e + c], lda = KB x points, self pairs

@@ -1317,8 +1317,9 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     NearArgs ra = na;  // outputs as requested by this call
     ra.dostrain_src = sa.dostrain_src;
     ra.dostrain_tgt = sa.dostrain_tgt;
-    launch_near_replay(st_, ra, near_base_.get(), near_ntri_.get(), store_K_, 1, ssl_s_.get(), sdl_s_.get(),
-                       store_.get());
+    build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+    launch_near_replay_batch(st_, ra, nntask_, ntask_.get(), 1, sa.dostrain_src, ssl_s_.get(),
+                             sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   }
   EFMM_CUDA_TRY(cudaEventRecord(ev_[7], st_));
   if (do_src) {
@@ -2094,7 +2095,6 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
     tedge_.resize(n);
     launch_tri_edge_prep(st_, n, tri_s_.get(), nullptr, nullptr, 0, 0, tedge_.get());
   }
-  if (mode) build_chunks(do_src, do_tgt);
   NearArgs na;
   na.nleaf = nnear_;
   na.leaves = near_leaves_.get(); na.nb_start = near_start_.get(); na.nb_items = near_items_.get();
@@ -2130,7 +2130,8 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
       build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
       launch_near_batch(st_, na, nntask_, ntask_.get(), R, (ds_src || ds_tgt) ? 1 : 0, ssl_s_.get(), sdl_s_.get(), n, nt);
     } else {
-      launch_near_replay_batch(st_, na, nchunk_, chunk_leaf_.get(), chunk_e0_.get(), R, (ds_src || ds_tgt) ? 1 : 0,
+      build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+      launch_near_replay_batch(st_, na, nntask_, ntask_.get(), R, (ds_src || ds_tgt) ? 1 : 0,
                                ssl_s_.get(), sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
     }
   }
@@ -2557,7 +2558,7 @@ void Plan::build_near_tasks(int do_src, int do_tgt, int pts) {
     for (int q = 0; q < parts; q++) {
       const int cnt = (int)((long long)nt * (q + 1) / parts - (long long)nt * q / parts);
       for (int e0 = 0; e0 < nep; e0 += cs) {
-        const NearTask t{(int)i, e0, std::min(cs, nep - e0), r, k, cnt, parts > 1};
+        const NearTask t{(int)i, e0, std::min(cs, nep - e0), r, k, (int)((long long)nt * q / parts), cnt, parts > 1};
         ((long long)t.ne * cnt * 2 >= W ? big : small).push_back(t);
       }
       for (k += cnt; r < near_rstart_h_[i + 1] && k >= near_rng_h_[r].y; r++) k -= near_rng_h_[r].y;
@@ -2933,8 +2934,8 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   rec(6);
   // near field: refined quadrature of the whole image kernel, stored, then
   // contracted with the right-hand sides
-  build_chunks(0, 1);
   if (store_now) {
+    build_chunks(0, 1);
     HsStoreArgs ha;
     ha.leaves = near_leaves_.get(); ha.nb_start = near_start_.get(); ha.nb_items = near_items_.get();
     ha.box_src_start = tr_.sstart.get(); ha.box_src_count = tr_.scount.get();
@@ -2963,7 +2964,8 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   na.do_src = 0; na.do_tgt = 1;
   na.rlam = rlam; na.rmu = rmu;
   na.u_src = nullptr; na.e_src = nullptr; na.u_tgt = ut_s_.get(); na.e_tgt = et_s_.get();
-  launch_near_replay_batch(st_, na, nchunk_, chunk_leaf_.get(), chunk_e0_.get(), R, dstr, ssl_s_.get(), sdl_s_.get(),
+  build_near_tasks(0, 1, NEAR_BATCH_PTS);
+  launch_near_replay_batch(st_, na, nntask_, ntask_.get(), R, dstr, ssl_s_.get(), sdl_s_.get(),
                            n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   rec(7);
   k_scatter_out<<<dim3((nt + 255) / 256, R), 256, 0, st_>>>(nt, tr_.izt.get(), ut_s_.get(), et_s_.get(), d_u_tgt,
