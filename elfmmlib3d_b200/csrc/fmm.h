@@ -80,6 +80,13 @@ struct L2TArgs {
 // (the products' 16-byte copies in FP32 and FP64).
 __host__ __device__ inline long long l2t_ld(int P) { return (9LL * P + 3) & ~3LL; }
 
+// P2M of R (few) right-hand sides on the FP64 tensor cores (leaf_mma.cu), the
+// free-space passes (columns 4r + pass of C per box) or the image columns
+// (layout of launch_p2m_img); T = double ADDS to zeroed expansions, float
+// stores the normalised basis.  Returns false (nothing launched) when the
+// order is too high for its tiles.
+template <class T, bool IMG>
+bool launch_p2m_mma(cudaStream_t st, int nleaf, const P2MArgs& a, int R, long long ubase, T* mpole);
 void launch_build_ops(cudaStream_t st, int nop, const OpDesc* ops, double* mats, int maxp);
 void launch_p2m(cudaStream_t st, int nleaf, const P2MArgs& a, int nrhs = 1);
 // P2M of R right-hand sides as a product (columns 4R per box); writes mpole
