@@ -2275,6 +2275,7 @@ __global__ void k_l2t_finish_img(const L2TArgs a, int R, const int* __restrict__
 }
 
 bool launch_l2t_img(cudaStream_t st, int nleaf, const L2TArgs& a, int R, long long ubase) {
+  if (launch_l2t_mma(st, nleaf, a, R, ubase, true)) return true;  // orders above: the kernel here
   const size_t smem = sizeof(double) * 7 * 2 * (size_t)ncoef(a.p) + sizeof(cplx) * L2T_WARPS * ncoef(a.p);
   if (smem > 227 * 1024) return false;  // high orders: the two-stage form
   if (nleaf <= 0 || R <= 0) return true;
@@ -2559,6 +2560,7 @@ template void launch_translate<float>(cudaStream_t, int, const TransTask*, const
 
 void launch_l2t(cudaStream_t st, int nleaf, const L2TArgs& a, int nrhs) {
   if (nleaf <= 0) return;
+  if (launch_l2t_mma(st, nleaf, a, nrhs, 0, false)) return;  // orders above: the kernel here
   int nw = L2T_WARPS;
   auto need = [&](int w) {
     return sizeof(double) * 4 * 2 * (size_t)ncoef(a.p) + sizeof(cplx) * w * (size_t)ncoef(a.p);

@@ -87,6 +87,9 @@ __host__ __device__ inline long long l2t_ld(int P) { return (9LL * P + 3) & ~3LL
 // order is too high for its tiles.
 template <class T, bool IMG>
 bool launch_p2m_mma(cudaStream_t st, int nleaf, const P2MArgs& a, int R, long long ubase, T* mpole);
+// L2T of R (few) right-hand sides likewise: free-space columns 4r + pass of C
+// per box, or the image columns (layout of launch_l2t_img).
+bool launch_l2t_mma(cudaStream_t st, int nleaf, const L2TArgs& a, int R, long long ubase, bool image);
 void launch_build_ops(cudaStream_t st, int nop, const OpDesc* ops, double* mats, int maxp);
 void launch_p2m(cudaStream_t st, int nleaf, const P2MArgs& a, int nrhs = 1);
 // P2M of R right-hand sides as a product (columns 4R per box); writes mpole

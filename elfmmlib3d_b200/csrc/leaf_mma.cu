@@ -34,7 +34,12 @@
 // half-space fault of 49,950 triangles, free-space 7.5 -> 1.5 and image columns
 // 14.8 -> 4.7 ms; 1,702 triangles, image 7.4 -> 0.27 ms.  16 warps of 6 row
 // tiles instead of 8 of 12 at order 26: 9.4 against 8.7 ms on the large case.
-// @MEASURED@
+// L2T measured likewise, against a warp per point with lanes over the (n, m)
+// terms (k_l2t, k_l2t_img): 577,687 points 25.9 -> 7.9 ms, the fault 9.0 -> 1.3
+// ms (both plans), 81,920 + 62,501 points (mixed form) 6.4 -> 1.9 ms; the
+// image columns of 2,003 points in 52 leaves 3.2 -> 0.09 ms (0.42 with one CTA
+// per leaf); 18,034 triangles at order 39 (8 points per chunk), two
+// right-hand sides, image columns 12.6 -> 2.3 ms.
 #include <algorithm>
 
 #include "common.cuh"
@@ -369,5 +374,230 @@ template bool launch_p2m_mma<double, false>(cudaStream_t, int, const P2MArgs&, i
 template bool launch_p2m_mma<float, false>(cudaStream_t, int, const P2MArgs&, int, long long, float*);
 template bool launch_p2m_mma<double, true>(cudaStream_t, int, const P2MArgs&, int, long long, double*);
 template bool launch_p2m_mma<float, true>(cudaStream_t, int, const P2MArgs&, int, long long, float*);
+
+// ------------------------------------------------------------------------ L2T
+// Functionals v of a column (value, d_z, d_zz, the real and imaginary parts of
+// d_x + i d_y, of that of d_z, and of (d_x + i d_y)^2): shifts a in n and b in
+// m, sign, imaginary part.
+struct LmTerm {
+  int a, b, sg, im;
+};
+__constant__ LmTerm c_lm_terms[9] = {{0, 0, 1, 0},  {1, 0, 1, 0},  {2, 0, 1, 0}, {1, 1, -1, 0}, {1, 1, -1, 1},
+                                     {2, 1, -1, 0}, {2, 1, -1, 1}, {2, 2, 1, 0}, {2, 2, 1, 1}};
+
+// The expansion rows extended for the shifts: degree N = 0..p + 2 (zero past
+// p), orders -2..N, entry N (N + 5) / 2 + M + 2 of a column.
+__host__ __device__ constexpr int lm_ext_size(int p) { return (p + 3) * (p + 8) / 2; }
+
+// Doubles of the harmonics of a chunk, or of the 16 warps' sums and their
+// total in their place.
+__host__ __device__ inline int lm_l2t_y(int p, int nb, int ncol) {
+  const int y = 2 * lm_plane_rows(ncoef(p)) * nb, w = 17 * nb * ncol;
+  return y > w ? y : w;
+}
+
+// One CTA per (leaf, right-hand side, part of the leaf's points), points in
+// chunks of NB, 16 warps splitting the product's rows; 9 outputs of a point by
+// 9 threads.
+template <int NB, bool IMG>
+__global__ void __launch_bounds__(512, 1)
+k_l2t_mma(const L2TArgs a, int R, long long ubase) {
+  constexpr int NW = 16, NTH = NW * 32, NQ = IMG ? 7 : 4, NTL = (9 * NQ + 7) / 8, NC = 8 * NTL, MT = NB / 8;
+  extern __shared__ __align__(16) double lm_sm[];
+  const int box = a.leaves[blockIdx.x], r = blockIdx.y;
+  const int sn = a.do_src ? a.scount[box] : 0, tn = a.do_tgt ? a.tcount[box] : 0, np = sn + tn;
+  if ((int)blockIdx.z * NB >= np) return;
+  const int p = a.p, nc = ncoef(p), D = 2 * nc, ncp = lm_plane_rows(nc), ext = lm_ext_size(p);
+  double* Y = lm_sm;                                  // [2 ncp][NB], later the warps' sums [NW][NB][NC]
+  double2* L = reinterpret_cast<double2*>(Y + lm_l2t_y(p, NB, NC));  // [NQ][ext]
+  double* S = Y + (size_t)NW * NB * NC;                 // [NB][NC]
+  double2* tab = L + NQ * ext;
+  unsigned short* nm = reinterpret_cast<unsigned short*>(tab + nc);  // [ncp]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lev = a.level[box];
+  const double s = a.size / (double)(1ull << lev), is = 1.0 / s, is2 = is * is;
+  double c[3];
+  for (int d = 0; d < 3; d++) c[d] = a.c0[d] - a.size / 2 + (a.ijk[3 * box + d] - 1) * s + s / 2;
+  double org[3];
+  lame_origin(a.ijk, a.level, box, a.c0, a.size, a.flev, org);
+  harmonic_table(p, tab, nm);
+  for (int q = nc + tid; q < ncp; q += NTH) nm[q] = 0xffff;  // padding rows
+  // the extended expansion: thread (column, entry)
+  for (int N = warp; N <= p + 2; N += NW)
+    for (int i = lane; i < N + 3; i += 32) {
+      const int M = i - 2, am = M < 0 ? -M : M;
+      const bool in = N <= p && am <= N;
+      const int k = 2 * (N * (N + 1) / 2 + am);
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        double2 v = make_double2(0.0, 0.0);
+        if (in) {
+          const double* src = IMG ? (q < 6 ? a.local + ((size_t)box * 6 * R + (size_t)q * R + r) * D
+                                           : a.local + ubase + ((size_t)box * R + r) * D)
+                                  : a.local + ((size_t)box * a.C + 4 * r + q) * D;
+          v = *reinterpret_cast<const double2*>(src + k);
+          if (M < 0) {
+            if (am & 1) v.x = -v.x;
+            else v.y = -v.y;
+          }
+        }
+        L[q * ext + N * (N + 5) / 2 + i] = v;
+      }
+    }
+  // this lane's columns: offset of the column in L, shifts, signs of the two
+  // terms for even (re) and odd (im) rows are resolved per row below
+  const int lk = lane & 3, ln = lane >> 2;
+  int ta[NTL], tb[NTL], tim[NTL], tq[NTL];
+  double tsg[NTL];
+#pragma unroll
+  for (int j = 0; j < NTL; j++) {
+    const int col = 8 * j + ln, q = col / 9, v = col % 9;
+    const LmTerm t = c_lm_terms[v];
+    ta[j] = t.a;
+    tb[j] = t.b;
+    tim[j] = t.im;
+    tq[j] = q < NQ ? q * ext : 0;
+    tsg[j] = q < NQ ? (double)t.sg : 0.0;
+  }
+  const int s0 = a.sstart[box], t0 = a.tstart[box];
+  const int nks = 2 * ncp / 4;
+  for (int e0 = blockIdx.z * NB; e0 < np; e0 += gridDim.z * NB) {
+    __syncthreads();  // tables and L are there; the last chunk's sums are read
+    if (NB == 16 || (lane & 15) < NB) {
+      const int pt = lane & (NB - 1), e = min(e0 + pt, np - 1);
+      const double* X = e < sn ? a.src_pts + 3 * (size_t)(s0 + e) : a.tgt_pts + 3 * (size_t)(t0 + e - sn);
+      const double z[3] = {(X[0] - c[0]) * is, (X[1] - c[1]) * is, (X[2] - c[2]) * is};
+      harmonics_to<NB>(Y, tab, p, z, pt, 2 * warp + (lane >> 4), 2 * NW, ncp * NB);
+    }
+    __syncthreads();
+    double acc[MT][NTL][2];
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int j = 0; j < NTL; j++) acc[i][j][0] = acc[i][j][1] = 0.0;
+    // k steps of 4 rows of one part: the re rows first, then the im rows
+#pragma unroll 1
+    for (int ks = warp; ks < nks; ks += NW) {
+      const int row = 4 * ks + lk, part = 4 * ks >= ncp, cc = row - (part ? ncp : 0);
+      const int n = nm[cc] >> 8, m = nm[cc] & 255;
+      const bool in = nm[cc] != 0xffff;
+      // Y past the last coefficient is not there: its operand is zero too
+      double av[MT];
+#pragma unroll
+      for (int i = 0; i < MT; i++)
+        av[i] = in ? Y[row * NB + (((8 * i + ln) ^ ((cc & 3) << 2)) & (NB - 1))] : 0.0;
+      const double f = m == 0 ? 0.5 : 1.0;
+#pragma unroll
+      for (int j = 0; j < NTL; j++) {
+        double b = 0.0;
+        if (in) {
+          const int N = n + ta[j];
+          const double2* l = L + tq[j] + N * (N + 5) / 2 + m + 2;
+          const double2 x = l[tb[j]], z = l[-tb[j]];
+          const bool im = (part ^ tim[j]) != 0;
+          const double xv = im ? x.y : x.x, zv = im ? z.y : z.x;
+          // im = 0: x -+ z (minus for b = 1); im = 1, re rows: x + z for b = 1, x - z for b = 2;
+          // im = 1, im rows: -x - z for b = 1, -x + z for b = 2
+          const bool neg = tim[j] ? ((tb[j] == 1) == (part != 0)) : tb[j] == 1;
+          b = tsg[j] * f * ((tim[j] && part ? -xv : xv) + (neg ? -zv : zv));
+        }
+#pragma unroll
+        for (int i = 0; i < MT; i++) dmma(acc[i][j], av[i], b);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < MT; i++)
+#pragma unroll
+      for (int j = 0; j < NTL; j++)
+        *reinterpret_cast<double2*>(Y + ((size_t)warp * NB + 8 * i + ln) * NC + 8 * j + 2 * lk) =
+            make_double2(acc[i][j][0], acc[i][j][1]);
+    __syncthreads();
+    for (int q = tid; q < NB * NC; q += NTH) {
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < NW; w++) v += Y[(size_t)w * NB * NC + q];
+      S[q] = v;
+    }
+    __syncthreads();
+    // recombination: thread (point, output)
+    for (int q = tid; q < 9 * NB; q += NTH) {
+      const int pt = q % NB, o = q / NB, e = e0 + pt;
+      if (e >= np) continue;
+      const bool is_src = e < sn;
+      const int pidx = is_src ? s0 + e : t0 + (e - sn);
+      if (o >= 3 && !(is_src ? a.dostrain_src : a.dostrain_tgt)) continue;
+      const double* X = is_src ? a.src_pts + 3 * (size_t)pidx : a.tgt_pts + 3 * (size_t)pidx;
+      const double x[3] = {X[0], X[1], X[2]};
+      const double* Sp = S + (size_t)pt * NC;
+      auto grad = [&](int k, int i) { return is * Sp[9 * k + (i == 2 ? 1 : 3 + i)]; };
+      auto hess = [&](int k, int i, int j) {
+        const double* v = Sp + 9 * k;
+        const int ij = i + j;
+        double h;
+        if (i == j) h = i == 2 ? v[2] : 0.5 * ((i == 0 ? v[7] : -v[7]) - v[2]);
+        else h = ij == 1 ? 0.5 * v[8] : (ij == 2 ? v[5] : v[6]);
+        return is2 * h;
+      };
+      const double c1 = a.c1, al = a.alpha, imu = IMG ? 1.0 / a.mu : 0.0, sc = IMG ? (1.0 - al) / al : 0.0, x3 = -x[2];
+      if (o < 3) {
+        double u = (2.0 - c1) * Sp[9 * o] + grad(3, o);
+        for (int j = 0; j < 3; j++) u -= c1 * (x[j] - org[j]) * grad(j, o);
+        if (IMG) {
+          const double Pv = o < 2 ? grad(4, o) : -grad(4, 2) - (2.0 - al) * Sp[9 * 5];
+          u += sc * imu * grad(6, o) + x3 * imu * Pv;
+        }
+        ((is_src ? a.u_src : a.u_tgt) + 3 * ((is_src ? a.nsrc : a.ntgt) * (long long)r + pidx))[o] += u;
+      } else {
+        auto G = [&](int i, int b) {  // d u_i / d x_b (image: d u_i / d xb_b)
+          double v = (2.0 - c1) * grad(i, b) - c1 * grad(b, i) + hess(3, i, b);
+          for (int j = 0; j < 3; j++) v -= c1 * (x[j] - org[j]) * hess(j, i, b);
+          if (IMG) {
+            v += sc * imu * hess(6, i, b);
+            const double dP = i < 2 ? hess(4, i, b) : -hess(4, 2, b) - (2.0 - al) * grad(5, b);
+            const double Pv = i < 2 ? grad(4, i) : -grad(4, 2) - (2.0 - al) * Sp[9 * 5];
+            v += imu * ((b == 2 ? -Pv : 0.0) + x3 * dP);
+          }
+          return v;
+        };
+        const int k = o - 3, i = k < 3 ? k : (k == 5 ? 1 : 0), j = k < 3 ? k : (k == 3 ? 1 : 2);
+        double v;
+        if (i == j) v = IMG && i == 2 ? -G(2, 2) : G(i, i);
+        else v = 0.5 * ((IMG && j == 2 ? -G(i, j) : G(i, j)) + G(j, i));
+        ((is_src ? a.e_src : a.e_tgt) + 6 * ((is_src ? a.nsrc : a.ntgt) * (long long)r + pidx))[k] += v;
+      }
+    }
+  }
+}
+
+static size_t l2t_mma_smem(int p, int nb, bool img) {
+  const int nq = img ? 7 : 4, ncol = 8 * ((9 * nq + 7) / 8), nc = ncoef(p);
+  return 8 * ((size_t)lm_l2t_y(p, nb, ncol) + 2 * (size_t)nq * lm_ext_size(p) + 2 * (size_t)nc) +
+         2 * (size_t)lm_plane_rows(nc) + 8;
+}
+
+bool launch_l2t_mma(cudaStream_t st, int nleaf, const L2TArgs& a, int R, long long ubase, bool image) {
+  const int nb = l2t_mma_smem(a.p, 16, image) <= 227 * 1024 ? 16 : 8;
+  const size_t smem = l2t_mma_smem(a.p, nb, image);
+  if (smem > 227 * 1024) return false;
+  if (nleaf <= 0 || R <= 0) return true;
+  auto go = [&](auto kern) {
+    EFMM_CUDA_TRY(smem_raise(kern, (int)smem));
+    // parts while the leaves leave SMs without a CTA (the few, full leaves near
+    // the surface that hold an image plan's points)
+    const int parts = std::max(1, std::min(16, 2 * 148 / (nleaf * R)));
+    kern<<<dim3(nleaf, R, parts), 512, smem, st>>>(a, R, ubase);
+    count_launch();
+  };
+  if (image) {
+    if (nb == 16) go(k_l2t_mma<16, true>);
+    else go(k_l2t_mma<8, true>);
+  } else {
+    if (nb == 16) go(k_l2t_mma<16, false>);
+    else go(k_l2t_mma<8, false>);
+  }
+  EFMM_CUDA_TRY(cudaGetLastError());
+  return true;
+}
 
 }  // namespace efmm
