@@ -25,10 +25,10 @@ struct TreeDev {
 struct TreeScratch {
   DevBuf<char> tmp;
   DevBuf<double> bb;
-  DevBuf<int> pbs, pbt, izs2, izt2, split, cs, ct, nch, off;
-  DevBuf<unsigned long long> ks, ks2, kt, kt2, k0, k1;
-  DevBuf<int> l2cnt, l2off, l2items, c1, c3, o1, o3, cnt, v0;
-  DevBuf<int2> pairs, p1, p3, p4;
+  DevBuf<int> pbs, pbt, izs2, izt2, split, cs, ct, nch, off, info;
+  DevBuf<unsigned char> ds, dt;        // digit of every point
+  DevBuf<unsigned long long> ks, ks2;  // keys of the radix path
+  DevBuf<int> cnt, cur, u1, u3, u4;    // row counts, cursors and unsorted rows of the lists
 };
 
 // Box ids are 0-based; ijk are the reference's 1-based grid indices; point
