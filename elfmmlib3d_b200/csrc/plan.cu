@@ -80,32 +80,147 @@ __global__ void k_gather(int n, int w, const int* __restrict__ perm, const doubl
   size_t r = (size_t)blockIdx.y * w * n;  // right-hand side blockIdx.y
   for (int c = 0; c < w; c++) out[r + (size_t)w * i + c] = in[r + (size_t)w * j + c];
 }
-// M2L pairs of list 2: pass 0 counts per operator group, pass 1 places
-// (src box, dst box, 1/s) at the group's cursor
-__global__ void k_m2l_pairs(int nb, int pass, const int* __restrict__ level, const int* __restrict__ ijk,
-                            const int* __restrict__ scount, const int* __restrict__ tcount,
-                            const int* __restrict__ l2s, const int* __restrict__ l2i, const int* __restrict__ m2lg,
-                            double size, int* __restrict__ cnt, int* __restrict__ cursor,
-                            TransPair* __restrict__ out) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= nb) return;
-  if (level[b] < 2 || scount[b] + tcount[b] == 0) return;
-  const double inv_s = (double)(1ull << level[b]) / size;
-  for (int q = l2s[b]; q < l2s[b + 1]; q++) {
-    const int sb = l2i[q];
-    if (scount[sb] == 0) continue;
-    const int di = ijk[3 * b] - ijk[3 * sb], dj = ijk[3 * b + 1] - ijk[3 * sb + 1],
-              dk = ijk[3 * b + 2] - ijk[3 * sb + 2];
-    if (di < -3 || di > 3 || dj < -3 || dj > 3 || dk < -3 || dk > 3) continue;  // not a list-2 offset
-    const int g = m2lg[(di + 3) * 49 + (dj + 3) * 7 + (dk + 3)];
-    if (g < 0) continue;
-    if (pass == 0) {
-      atomicAdd(&cnt[g], 1);
+// Offset code 0..342 of a list-2 pair (source box sb, box b), -1 if it has none
+__device__ __forceinline__ int m2l_code(const int* __restrict__ ijk, int b, int sb) {
+  const int di = ijk[3 * b] - ijk[3 * sb], dj = ijk[3 * b + 1] - ijk[3 * sb + 1], dk = ijk[3 * b + 2] - ijk[3 * sb + 2];
+  if (di < -3 || di > 3 || dj < -3 || dj > 3 || dk < -3 || dk > 3) return -1;
+  return (di + 3) * 49 + (dj + 3) * 7 + (dk + 3);
+}
+
+// M2L pairs of list 2 by offset: FILL = false counts them, FILL = true places
+// (src box, dst box, 1/s) from the offset's cursor on (-1: no operator).  A
+// warp walks the rows of M2L_BOXES / 8 boxes, the CTA counts in shared memory
+// and takes each offset's places with one atomic: bound by the rows' scattered
+// loads, 19 us for both passes on 4,500 boxes and 158,000 pairs (92 with a
+// thread per box and an atomic per pair).
+constexpr int M2L_BOXES = 32;
+template <bool FILL>
+__global__ void __launch_bounds__(256)
+k_m2l_pairs(int nb, const int* __restrict__ level, const int* __restrict__ ijk, const int* __restrict__ scount,
+            const int* __restrict__ tcount, const int* __restrict__ l2s, const int* __restrict__ l2i, double size,
+            int* __restrict__ cur, TransPair* __restrict__ out) {
+  __shared__ int cnt[343];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b0 = blockIdx.x * M2L_BOXES;
+  auto walk = [&](auto visit) {
+    for (int b = b0 + warp; b < min(nb, b0 + M2L_BOXES); b += 8) {
+      if (level[b] < 2 || scount[b] + tcount[b] == 0) continue;
+      for (int q = l2s[b] + lane; q < l2s[b + 1]; q += 32) {
+        const int sb = l2i[q];
+        if (scount[sb] == 0) continue;
+        const int o = m2l_code(ijk, b, sb);
+        if (o >= 0) visit(b, sb, o);
+      }
+    }
+  };
+  for (int o = threadIdx.x; o < 343; o += 256) cnt[o] = 0;
+  __syncthreads();
+  walk([&](int, int, int o) { atomicAdd(&cnt[o], 1); });
+  __syncthreads();
+  for (int o = threadIdx.x; o < 343; o += 256) {
+    if (!FILL) {
+      if (cnt[o]) atomicAdd(&cur[o], cnt[o]);
     } else {
-      const int pos = atomicAdd(&cursor[g], 1);
-      out[pos] = TransPair{sb, b, inv_s};
+      cnt[o] = cnt[o] && cur[o] >= 0 ? atomicAdd(&cur[o], cnt[o]) : -1;
     }
   }
+  if (!FILL) return;
+  __syncthreads();
+  walk([&](int b, int sb, int o) {
+    if (cnt[o] < 0) return;
+    out[atomicAdd(&cnt[o], 1)] = TransPair{sb, b, (double)(1ull << level[b]) / size};
+  });
+}
+
+// What the host needs to know of a box to cut the work
+struct BoxInfo {
+  int parent, kids, sc, tc;   // kids: number | octant within the parent << 4
+  int nit, nrg, ntri, level;  // near list of a leaf: source boxes, ranges of adjoining triangles, triangles
+};
+
+// Near field of leaf b (one warp): the source boxes of list 1, itself, list 3
+// and list 4 of itself and its ancestors (ITER pairing,
+// src/elfmm3dtria_iter_1.f:1188-1225, read from the target side), and their
+// triangles as ranges, consecutive boxes that adjoin merged.  FILL = false
+// returns the counts; FILL = true writes boxes and ranges.
+template <bool FILL>
+__device__ __forceinline__ int3 near_row(int b, const int* __restrict__ parent, const int* __restrict__ sstart,
+                                         const int* __restrict__ scount, const int* __restrict__ l1s,
+                                         const int* __restrict__ l1i, const int* __restrict__ l3s,
+                                         const int* __restrict__ l3i, const int* __restrict__ l4s,
+                                         const int* __restrict__ l4i, int* __restrict__ items,
+                                         int2* __restrict__ rng) {
+  const int lane = threadIdx.x & 31;
+  const unsigned below = (1u << lane) - 1u;
+  int ni = 0, nr = 0, nt = 0, pend = -1;  // boxes, ranges, triangles so far; end of the last box
+  auto add = [&](const int* row, int n) {
+    for (int q0 = 0; q0 < n; q0 += 32) {
+      const int q = q0 + lane, s = q < n ? (row ? row[q] : b) : -1;
+      const int cnt = s >= 0 ? scount[s] : 0, st = cnt > 0 ? sstart[s] : 0;
+      const unsigned keep = __ballot_sync(0xffffffffu, cnt > 0);
+      const int prev = 31 - __clz(keep & below);  // -1: none in this chunk
+      const int pe = __shfl_sync(0xffffffffu, st + cnt, max(prev, 0));
+      const bool first = cnt > 0 && (prev >= 0 ? pe : pend) != st;
+      const unsigned fm = __ballot_sync(0xffffffffu, first);
+      if (FILL) {
+        const int r = nr + __popc(fm & (below | (1u << lane))) - 1;
+        if (cnt > 0) items[ni + __popc(keep & below)] = s;
+        if (first) rng[r] = make_int2(st, 0);
+        __syncwarp();
+        if (cnt > 0) atomicAdd(&rng[r].y, cnt);
+        __syncwarp();
+      }
+      if (keep) pend = __shfl_sync(0xffffffffu, st + cnt, 31 - __clz(keep));
+      ni += __popc(keep);
+      nr += __popc(fm);
+      nt += __reduce_add_sync(0xffffffffu, cnt);
+    }
+  };
+  add(l1i + l1s[b], l1s[b + 1] - l1s[b]);
+  add(nullptr, 1);
+  add(l3i + l3s[b], l3s[b + 1] - l3s[b]);
+  for (int a = b; a >= 0; a = parent[a]) add(l4i + l4s[a], l4s[a + 1] - l4s[a]);
+  return make_int3(ni, nr, nt);
+}
+
+// A warp per box (FILL = false: its record) or per leaf i of the near field
+// (FILL = true).  Bound by the chain of row loads per warp: 7 us each for the
+// 4,500 boxes of 20,480 triangles, where host loops over copies of the lists
+// took 1.25 ms; for 327,680 triangles they took 24 ms of set_geometry, now 1.9.
+template <bool FILL>
+__global__ void __launch_bounds__(128)
+k_near_rows(int n, const int* __restrict__ leaves, const int* __restrict__ level, const int* __restrict__ ijk,
+            const int* __restrict__ parent, const int* __restrict__ nkids, const int* __restrict__ sstart,
+            const int* __restrict__ scount, const int* __restrict__ tcount, const int* __restrict__ l1s,
+            const int* __restrict__ l1i, const int* __restrict__ l3s, const int* __restrict__ l3i,
+            const int* __restrict__ l4s, const int* __restrict__ l4i, BoxInfo* __restrict__ info,
+            const int* __restrict__ start, const int* __restrict__ rstart, int* __restrict__ items,
+            int2* __restrict__ rng) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= n) return;
+  if (FILL) {
+    near_row<true>(leaves[i], parent, sstart, scount, l1s, l1i, l3s, l3i, l4s, l4i, items + start[i],
+                   rng + rstart[i]);
+    return;
+  }
+  int3 c = make_int3(0, 0, 0);
+  if (nkids[i] == 0 && scount[i] + tcount[i] > 0)
+    c = near_row<false>(i, parent, sstart, scount, l1s, l1i, l3s, l3i, l4s, l4i, nullptr, nullptr);
+  if (lane == 0) {
+    const int oct = ((ijk[3 * i] - 1) & 1) + 2 * ((ijk[3 * i + 1] - 1) & 1) + 4 * ((ijk[3 * i + 2] - 1) & 1);
+    info[i] = BoxInfo{parent[i], nkids[i] | oct << 4, scount[i], tcount[i], c.x, c.y, c.z, level[i]};
+  }
+}
+
+// first range and offset of every near-field work item, from its first triangle p0
+__global__ void k_near_seek(int n, const int* __restrict__ rstart, const int2* __restrict__ rng,
+                            NearTask* __restrict__ tasks) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const int li = tasks[i].li, end = rstart[li + 1];
+  int r = rstart[li], k = tasks[i].p0;
+  while (r < end && k >= rng[r].y) k -= rng[r++].y;
+  tasks[i].r0 = r;
+  tasks[i].k0 = k;
 }
 
 // user (R, n, 3) -> tree order, right-hand side innermost: out[(i*3+d)*R + r]
@@ -430,111 +545,83 @@ void Plan::build_worklists() {
     fprintf(stderr, "build_worklists %-10s %8.2f ms\n", what, std::chrono::duration<double, std::milli>(t - tp).count());
     tp = t;
   };
-  int nb = tr_.nboxes;
-  auto level = d2h(tr_.level, nb, st_);
-  auto ijk = d2h(tr_.ijk, 3 * (size_t)nb, st_);
-  auto parent = d2h(tr_.parent, nb, st_);
-  auto nkids = d2h(tr_.nkids, nb, st_);
-  auto kids = d2h(tr_.kids, 8 * (size_t)nb, st_);
-  auto scount = d2h(tr_.scount, nb, st_);
-  auto tcount = d2h(tr_.tcount, nb, st_);
-  auto csr = [&](const DevBuf<int>& s, const DevBuf<int>& it, std::vector<int>& hs, std::vector<int>& hi) {
-    hs = d2h(s, nb + 1, st_);
-    hi = d2h(it, hs[nb], st_);
+  const int nb = tr_.nboxes;
+  // one record per box and the M2L pairs per offset: the only copies to the host
+  box_info_.resize(nb);
+  m2l_cnt_.resize(344);
+  m2l_cnt_.zero(st_);
+  auto near_rows = [&](auto fill, int n, const int* leaves, int* items, int2* rng) {
+    k_near_rows<decltype(fill)::value><<<(n + 3) / 4, 128, 0, st_>>>(
+        n, leaves, tr_.level.get(), tr_.ijk.get(), tr_.parent.get(), tr_.nkids.get(), tr_.sstart.get(),
+        tr_.scount.get(), tr_.tcount.get(), tr_.l1_start.get(), tr_.l1_items.get(), tr_.l3_start.get(),
+        tr_.l3_items.get(), tr_.l4_start.get(), tr_.l4_items.get(), box_info_.get(), near_start_.get(),
+        near_rstart_.get(), items, rng); count_launch();
   };
-  std::vector<int> l1s, l1i, l2s, l2i, l3s, l3i, l4s, l4i;
-  csr(tr_.l1_start, tr_.l1_items, l1s, l1i);
-  csr(tr_.l2_start, tr_.l2_items, l2s, l2i);
-  csr(tr_.l3_start, tr_.l3_items, l3s, l3i);
-  csr(tr_.l4_start, tr_.l4_items, l4s, l4i);
-
+  auto m2l_by_offset = [&](auto fill, int* cur, TransPair* out) {
+    k_m2l_pairs<decltype(fill)::value><<<(nb + M2L_BOXES - 1) / M2L_BOXES, 256, 0, st_>>>(
+        nb, tr_.level.get(), tr_.ijk.get(), tr_.scount.get(), tr_.tcount.get(), tr_.l2_start.get(),
+        tr_.l2_items.get(), tr_.size, cur, out); count_launch();
+  };
+  near_rows(std::false_type(), nb, nullptr, nullptr, nullptr);
+  if (p_ > 0 && tr_.nlev >= 2) m2l_by_offset(std::false_type(), m2l_cnt_.get(), nullptr);
+  std::vector<BoxInfo> box(nb);
+  std::vector<int> m2l_cnt(343);
+  EFMM_CUDA_TRY(cudaMemcpyAsync(box.data(), box_info_.get(), nb * sizeof(BoxInfo), cudaMemcpyDeviceToHost, st_));
+  EFMM_CUDA_TRY(cudaMemcpyAsync(m2l_cnt.data(), m2l_cnt_.get(), 343 * sizeof(int), cudaMemcpyDeviceToHost, st_));
+  EFMM_CUDA_TRY(cudaStreamSynchronize(st_));
   mark("d2h");
-  // near field: per leaf with evaluation points, source boxes from
-  // list1 U self U list3 U list4(ancestors-or-self)  (ITER pairing,
-  // src/elfmm3dtria_iter_1.f:1188-1225, read from the target side)
-  std::vector<int> nleaves, nstart, nitems;
-  nstart.push_back(0);
-  for (int b = 0; b < nb; b++) {
-    if (nkids[b] != 0) continue;
-    if (scount[b] + tcount[b] == 0) continue;
-    size_t before = nitems.size();
-    auto add = [&](int s) {
-      if (scount[s] > 0) nitems.push_back(s);
-    };
-    for (int q = l1s[b]; q < l1s[b + 1]; q++) add(l1i[q]);
-    add(b);
-    for (int q = l3s[b]; q < l3s[b + 1]; q++) add(l3i[q]);
-    for (int a = b; a >= 0; a = parent[a])
-      for (int q = l4s[a]; q < l4s[a + 1]; q++) add(l4i[q]);
-    if (nitems.size() == before) continue;
-    nleaves.push_back(b);
-    nstart.push_back((int)nitems.size());
-  }
+  // near field: the leaves with evaluation points and near triangles
+  std::vector<int> nleaves, nstart(1, 0), nrstart(1, 0);
   near_sc_h_.clear();
   near_tc_h_.clear();
   near_ntri_h_.clear();
-  for (size_t i = 0; i < nleaves.size(); i++) {
-    int b = nleaves[i], nt = 0;
-    for (int q = nstart[i]; q < nstart[i + 1]; q++) nt += scount[nitems[q]];
-    near_sc_h_.push_back(scount[b]);
-    near_tc_h_.push_back(tcount[b]);
-    near_ntri_h_.push_back(nt);
+  near_pairs_ = 0;  // point pairs for the throughput model
+  for (int b = 0; b < nb; b++) {
+    const BoxInfo& x = box[b];
+    if (x.nit == 0) continue;
+    nleaves.push_back(b);
+    nstart.push_back(nstart.back() + x.nit);
+    nrstart.push_back(nrstart.back() + x.nrg);
+    near_sc_h_.push_back(x.sc);
+    near_tc_h_.push_back(x.tc);
+    near_ntri_h_.push_back(x.ntri);
+    near_pairs_ += (long long)(x.sc + x.tc) * x.ntri;
   }
+  nnear_ = (int)nleaves.size();
+  h2d(near_leaves_, nleaves, st_);
+  h2d(near_start_, nstart, st_);
+  h2d(near_rstart_, nrstart, st_);
   h2d(near_ntri_, near_ntri_h_, st_);
+  near_items_.resize(nstart.back());
+  near_rng_.resize(nrstart.back());
+  if (nnear_) near_rows(std::true_type(), nnear_, near_leaves_.get(), near_items_.get(), near_rng_.get());
   store_valid_ = false;
   store_gen_++;
   ntc_key_ = -1;
   chunk_key_ = -1;
-  near_pairs_ = 0;
-  {
-    // count point pairs for the throughput model
-    auto sst = d2h(tr_.sstart, nb, st_);
-    near_rng_h_.clear();
-    near_rstart_h_.assign(1, 0);
-    for (size_t i = 0; i < nleaves.size(); i++) {
-      int b = nleaves[i];
-      near_pairs_ += (long long)(scount[b] + tcount[b]) * near_ntri_h_[i];
-      // the list's triangles as ranges, consecutive boxes that adjoin merged
-      const size_t first = near_rng_h_.size();
-      for (int q = nstart[i]; q < nstart[i + 1]; q++) {
-        const int s = nitems[q];
-        if (near_rng_h_.size() > first && near_rng_h_.back().x + near_rng_h_.back().y == sst[s])
-          near_rng_h_.back().y += scount[s];
-        else
-          near_rng_h_.push_back(make_int2(sst[s], scount[s]));
-      }
-      near_rstart_h_.push_back((int)near_rng_h_.size());
-    }
-    h2d(near_rstart_, near_rstart_h_, st_);
-    h2d(near_rng_, near_rng_h_, st_);
-  }
   ntask_key_ = -1;
-  nnear_ = (int)nleaves.size();
-  h2d(near_leaves_, nleaves, st_);
-  h2d(near_start_, nstart, st_);
-  h2d(near_items_, nitems, st_);
 
   mark("near");
   // far field
   far_ = (p_ > 0) && (tr_.nlev >= 2);
   std::vector<int> p2m, l2t;
   for (int b = 0; b < nb; b++) {
-    if (nkids[b] != 0 || level[b] < 2) continue;
-    if (scount[b] > 0) p2m.push_back(b);
-    if (scount[b] + tcount[b] > 0) l2t.push_back(b);
+    if ((box[b].kids & 15) != 0 || box[b].level < 2) continue;
+    if (box[b].sc > 0) p2m.push_back(b);
+    if (box[b].sc + box[b].tc > 0) l2t.push_back(b);
   }
   if (p2m.empty()) far_ = false;
   np2m_ = (int)p2m.size();
   nl2t_ = (int)l2t.size();
   p2m_h_ = p2m;
   p2m_sc_h_.clear();
-  for (int b : p2m) p2m_sc_h_.push_back(scount[b]);
+  for (int b : p2m) p2m_sc_h_.push_back(box[b].sc);
   l2t_sc_h_.clear();
   l2t_tc_h_.clear();
   l2t_h_ = l2t;
   for (int b : l2t) {
-    l2t_sc_h_.push_back(scount[b]);
-    l2t_tc_h_.push_back(tcount[b]);
+    l2t_sc_h_.push_back(box[b].sc);
+    l2t_tc_h_.push_back(box[b].tc);
   }
   lchunk_key_ = -1;
   h2d(p2m_leaves_, p2m, st_);
@@ -544,7 +631,6 @@ void Plan::build_worklists() {
   l2l_.clear();
   if (!far_) return;
   ensure_ops();
-  const int* m2lg = ops_->m2l_group;
   const std::vector<int>& dims = ops_->dims;
   // group the pairs of one level by operator; one segment per group
   auto add_level = [&](std::vector<std::pair<int, TransPair>>& gp, std::vector<TransPair>& pairs,
@@ -567,58 +653,48 @@ void Plan::build_worklists() {
   m2m_.clear();
   m2l_.clear();
   l2l_.clear();
-  std::vector<TransPair> m2m_pairs, l2l_pairs, m2l_pairs;
+  std::vector<TransPair> m2m_pairs, l2l_pairs;
   mark("far-leaves");
   // M2M bottom-up: children at level lev -> parents at lev-1 (parents >= 2)
   for (int lev = tr_.nlev; lev >= 3; lev--) {
     std::vector<std::pair<int, TransPair>> gp;
     int lo = tr_.laddr[lev].first, cnt = tr_.laddr[lev].second;
     for (int b = lo; b < lo + cnt; b++) {
-      if (scount[b] == 0) continue;
-      int P = parent[b];
-      int dg = ((ijk[3 * b] - 1) & 1) + 2 * ((ijk[3 * b + 1] - 1) & 1) + 4 * ((ijk[3 * b + 2] - 1) & 1);
-      gp.push_back({ops_->m2m_group[dg], TransPair{b, P, 1.0}});
+      if (box[b].sc == 0) continue;
+      gp.push_back({ops_->m2m_group[box[b].kids >> 4], TransPair{b, box[b].parent, 1.0}});
     }
     add_level(gp, m2m_pairs, m2m_);
   }
   mark("m2m");
   // M2L: list 2 of every box at level >= 2, grouped by operator on the
-  // device (count per group, then fill; order within a group is arbitrary)
+  // device (order within a group is arbitrary)
   {
-    DevBuf<int>& cnt = m2l_cnt_;
-    cnt.resize(344);
-    cnt.zero(st_);
-    const int gb = (nb + 255) / 256;
-    k_m2l_pairs<<<gb, 256, 0, st_>>>(nb, 0, tr_.level.get(), tr_.ijk.get(), tr_.scount.get(), tr_.tcount.get(),
-                                     tr_.l2_start.get(), tr_.l2_items.get(), ops_->m2lg_dev.get(), tr_.size,
-                                     cnt.get(), nullptr, nullptr); count_launch();
-    std::vector<int> hc = d2h(cnt, 343, st_);
-    std::vector<int> start(344, 0);
-    for (int g = 0; g < 343; g++) start[g + 1] = start[g] + hc[g];
-    const int tot = start[343];
-    int s0 = (int)m2l_.segs.size();
-    for (int g = 0; g < 343; g++)
-      if (hc[g] > 0) m2l_.segs.push_back({g, start[g], hc[g]});
-    m2l_.lev.push_back({s0, (int)m2l_.segs.size() - s0});
-    h2d(m2l_cursor_, start, st_);
+    std::vector<int> at(343, -1), cursor(344, -1);  // offset of an operator; first place of an offset
+    for (int o = 0; o < 343; o++)
+      if (ops_->m2l_group[o] >= 0) at[ops_->m2l_group[o]] = o;
+    int tot = 0;
+    for (int g = 0; g < 343; g++) {
+      const int np = at[g] >= 0 ? m2l_cnt[at[g]] : 0;
+      if (np == 0) continue;
+      m2l_.segs.push_back({g, tot, np});
+      cursor[at[g]] = tot;
+      tot += np;
+    }
+    m2l_.lev.push_back({0, (int)m2l_.segs.size()});
+    h2d(m2l_cursor_, cursor, st_);
     m2l_.pairs.resize(std::max(tot, 1));
-    k_m2l_pairs<<<gb, 256, 0, st_>>>(nb, 1, tr_.level.get(), tr_.ijk.get(), tr_.scount.get(), tr_.tcount.get(),
-                                     tr_.l2_start.get(), tr_.l2_items.get(), ops_->m2lg_dev.get(), tr_.size,
-                                     nullptr, m2l_cursor_.get(), m2l_.pairs.get()); count_launch();
+    m2l_by_offset(std::true_type(), m2l_cursor_.get(), m2l_.pairs.get());
     m2l_pairs_h_ = tot;
   }
   mark("m2l");
   // L2L top-down: parents at level lev (>= 2) -> children
   for (int lev = 2; lev < tr_.nlev; lev++) {
     std::vector<std::pair<int, TransPair>> gp;
-    int lo = tr_.laddr[lev].first, cnt = tr_.laddr[lev].second;
-    for (int b = lo; b < lo + cnt; b++) {
-      for (int q = 0; q < nkids[b]; q++) {
-        int k = kids[8 * b + q];
-        if (scount[k] + tcount[k] == 0) continue;
-        int dg = ((ijk[3 * k] - 1) & 1) + 2 * ((ijk[3 * k + 1] - 1) & 1) + 4 * ((ijk[3 * k + 2] - 1) & 1);
-        gp.push_back({ops_->l2l_group[dg], TransPair{b, k, 1.0}});
-      }
+    int lo = tr_.laddr[lev + 1].first, cnt = tr_.laddr[lev + 1].second;
+    // (the boxes of a level are numbered by parent and octant)
+    for (int k = lo; k < lo + cnt; k++) {
+      if (box[k].sc + box[k].tc == 0) continue;
+      gp.push_back({ops_->l2l_group[box[k].kids >> 4], TransPair{box[k].parent, k, 1.0}});
     }
     add_level(gp, l2l_pairs, l2l_);
   }
@@ -2554,19 +2630,21 @@ void Plan::build_near_tasks(int do_src, int do_tgt, int pts) {
     if (nep == 0 || nt == 0) continue;
     const int nch = (nep + pts - 1) / pts, cs = (nep + nch - 1) / nch;
     const int parts = (int)std::min<long long>((nt + 15) / 16, ((long long)cs * nt + W - 1) / W);
-    int r = near_rstart_h_[i], k = 0;
     for (int q = 0; q < parts; q++) {
       const int cnt = (int)((long long)nt * (q + 1) / parts - (long long)nt * q / parts);
       for (int e0 = 0; e0 < nep; e0 += cs) {
-        const NearTask t{(int)i, e0, std::min(cs, nep - e0), r, k, (int)((long long)nt * q / parts), cnt, parts > 1};
+        const NearTask t{(int)i, e0, std::min(cs, nep - e0), 0, 0, (int)((long long)nt * q / parts), cnt, parts > 1};
         ((long long)t.ne * cnt * 2 >= W ? big : small).push_back(t);
       }
-      for (k += cnt; r < near_rstart_h_[i + 1] && k >= near_rng_h_[r].y; r++) k -= near_rng_h_[r].y;
     }
   }
   nntask_ = (int)(big.size() + small.size());
   big.insert(big.end(), small.begin(), small.end());
   h2d(ntask_, big, st_);
+  if (nntask_) {
+    k_near_seek<<<(nntask_ + 127) / 128, 128, 0, st_>>>(nntask_, near_rstart_.get(), near_rng_.get(), ntask_.get());
+    count_launch();
+  }
   ntask_key_ = key;
 }
 

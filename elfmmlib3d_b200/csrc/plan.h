@@ -368,8 +368,7 @@ class Plan {
   DevBuf<int> near_ntri_;
   DevBuf<int> near_rstart_;  // near triangles as ranges (NearArgs::rng)
   DevBuf<int2> near_rng_;
-  std::vector<int> near_rstart_h_;
-  std::vector<int2> near_rng_h_;
+  DevBuf<struct BoxInfo> box_info_;
   DevBuf<long long> near_base_;
   std::vector<long long> near_base_h_;
   // FP32 product-layout copy of the stored near field for mixed replays on
