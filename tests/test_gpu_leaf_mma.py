@@ -67,3 +67,33 @@ def test_image_few_equal_many(gpu, iprec, cells, nrhs):
     P.close()
     for a, b in zip(*outs):
         assert rel(a, b) < 1e-11
+
+
+@pytest.mark.parametrize("iprec,n,leaf", [(1, 777, 0), (2, 1280, 0), (2, 320, 1), (3, 1280, 0)])
+@pytest.mark.parametrize("nrhs", [1, 2, 3, 4])
+def test_mixed_few_right_hand_sides(gpu, iprec, n, leaf, nrhs):
+    """Mixed passes of few right-hand sides, on both sides of the line
+    between P2M one by one and the product form, are as close to the FP64
+    pass at the same orders as the same densities in a batch of 9, whose P2M
+    is the product form (half as much again allowed: FP32 rounding differs
+    with the order of the sums)."""
+    level = next(k for k in range(8) if 20 * 4 ** k >= n)
+    tri, nrm, cen = (a[:n] for a in G.sphere_triangles(level))
+    tgt = G.box_targets(61, 5)
+    rng = np.random.default_rng(n)
+    big = 9
+    ssl, sdl = rng.normal(size=(2, big, n, 3))
+    P = gpu.Plan(0)
+    P.set_mixed_floor(0.0)
+    if leaf:
+        assert P._L.efmm_plan_set_leaf(P._h, leaf) == 0
+    P.set_geometry(_dev(tri), _dev(nrm), _dev(cen), _dev(tgt), iprec=iprec)
+    assert P.info()["far"]
+    outs = []
+    for R, precision in ((nrhs, 1), (big, 1), (big, 0)):
+        o = [_zeros(R, n, 3), _zeros(R, n, 3, 3), _zeros(R, 61, 3), _zeros(R, 61, 3, 3)]
+        P.evaluate_batch(1.3, 0.7, R, _dev(ssl[:R]), _dev(sdl[:R]), *o, precision=precision)
+        outs.append([t[:nrhs].cpu().numpy() for t in o])
+    P.close()
+    for few, many, exact in zip(*outs):
+        assert 0 < rel(few, exact) <= 1.5 * rel(many, exact) < 1e-4
