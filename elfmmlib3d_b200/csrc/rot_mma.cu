@@ -23,12 +23,20 @@
 // Columns per CTA: 32 while the rows fit (p <= 28), else 16; fewer where a
 // launch's groups are so small that most of a tile would be padding.
 //
+// What bounds it is the FP64 tensor pipe and, between its bursts, the latency
+// of L2: a warp's next block has its first operator fragments loaded during
+// the last k step of the block before (across the barriers of the stages
+// too), and the sources of four staging steps are in flight together (two
+// cost 6 %); without both 29.7 ms instead of 25.5 on the first case below.
+// Atomics laid out so that a warp fills whole lines (half as many columns per
+// instruction) cost 6 %: the final pass is bound by instructions.
+//
 // Measured (all M2M + M2L + L2L launches of a pass) against full (re, im)
 // blocks on plain FP64 FMAs, 8 columns per CTA (bound by L2 latency): 327,680
 // triangles + 250,007 targets at iprec 2 (1.33 M box pairs x 4 columns) 78.5
-// -> 29.7 ms; 16 right-hand sides on 9,973 + 2,003 30.6 -> 11.2 ms (8.9e10
-// multiply-adds, 0.45 of the measured DGEMM rate, padding to 8 x 4 tiles not
-// counted); 20,011 particles 14.5 -> 4.7 ms; 20,480 triangles at iprec 1 3.9
+// -> 25.5 ms; 16 right-hand sides on 9,973 + 2,003 30.6 -> 10.0 ms (8.9e10
+// multiply-adds, 0.50 of the measured DGEMM rate, padding to 8 x 4 tiles not
+// counted); 20,011 particles 14.5 -> 4.6 ms; 20,480 triangles at iprec 1 3.9
 // -> 1.1 ms.
 #include <algorithm>
 #include <vector>
@@ -84,11 +92,23 @@ __device__ __forceinline__ void dmma(double* d, double a, double b) {
                : "d"(a), "d"(b));
 }
 
+// Operator fragments of a block's first k step, for up to RM_MT row tiles
+template <int NT>
+constexpr int RM_MT = NT == 4 ? 4 : 6;
+template <int NT>
+__device__ __forceinline__ void rm_first(double (&an)[RM_MT<NT>], const double* __restrict__ A, int mt, int lane) {
+#pragma unroll
+  for (int a = 0; a < RM_MT<NT>; a++)
+    if (a < mt) an[a] = __ldg(A + lane + 32 * a);
+}
+
 // One block of r <= 8 MT rows: stage 1 (shift) rows (m + i)^2 + m + part (m +
-// i), else rb + i; key of row i: kb + i.
+// i), else rb + i; key of row i: kb + i.  an holds its first fragments and
+// leaves with those of the warp's next block (An, mtn row tiles; none: 0).
 template <int MT, int NT>
 __device__ __forceinline__ void rm_block(double* __restrict__ X, const double* __restrict__ A, int r, bool shift,
-                                         int rb, int m, int part, int kb, int lane) {
+                                         int rb, int m, int part, int kb, int lane, double (&an)[RM_MT<NT>],
+                                         const double* __restrict__ An, int mtn) {
   constexpr int NC = 8 * NT;
   const int lk = lane & 3, ln = lane >> 2;
   auto row = [&](int i) {
@@ -102,9 +122,6 @@ __device__ __forceinline__ void rm_block(double* __restrict__ X, const double* _
     for (int b = 0; b < NT; b++) acc[a][b][0] = acc[a][b][1] = 0.0;
   const int kt = (r + 3) >> 2;
   const double* Al = A + lane;
-  double an[MT];
-#pragma unroll
-  for (int a = 0; a < MT; a++) an[a] = __ldg(Al + 32 * a);
   const int cx = ln ^ (((kb + lk) & 3) << 2);  // swizzled column of n-tile 0 in this lane's input rows
 #pragma unroll 2
   for (int k = 0; k < kt; k++) {
@@ -112,9 +129,12 @@ __device__ __forceinline__ void rm_block(double* __restrict__ X, const double* _
 #pragma unroll
     for (int a = 0; a < MT; a++) ac[a] = an[a];
     Al += 32 * MT;
-    if (k + 1 < kt)
+    if (k + 1 < kt) {
 #pragma unroll
       for (int a = 0; a < MT; a++) an[a] = __ldg(Al + 32 * a);
+    } else {
+      rm_first<NT>(an, An, mtn, lane);
+    }
     // rows past the block's last are met by zero operator columns
     const double* xr = X + (size_t)row(min(4 * k + lk, r - 1)) * NC;
 #pragma unroll
@@ -177,39 +197,61 @@ k_translate_mma(const TransTask* __restrict__ tasks, const TransPair* __restrict
   __syncthreads();
   const double* g0 = pool + op.base;
   const int nst = rm_stage(c_rm, p), ncg = (nc + 7) / 8;
-  // sources with Rz: lane (coefficient of 8, column of 4), both parts
-  for (int q = warp; q < ncg * (NC / 4); q += NW) {
-    const int c = (q % ncg) * 8 + (lane & 7), j = (q / ncg) * 4 + (lane >> 3);
-    if (c >= nc) continue;
-    const int n = nm[c] >> 8, m = nm[c] & 255;
-    const long long b = sb[j];
-    const double2 v = b >= 0 ? __ldg(reinterpret_cast<const double2*>(src + b) + c) : make_double2(0.0, 0.0);
-    const double2 R0 = __ldg(reinterpret_cast<const double2*>(g0 + 4 * m));
-    const double2 R1 = __ldg(reinterpret_cast<const double2*>(g0 + 4 * m + 2));
-    const int cs = (j ^ (((n + m) & 3) << 2)) & (NC - 1);
-    X[(size_t)(n * n + m) * NC + cs] = R0.x * v.x + R0.y * v.y;
-    if (m > 0) X[(size_t)(n * n + n + m) * NC + cs] = R1.x * v.x + R1.y * v.y;
-  }
   const unsigned char* list = sched + ((size_t)p * NW + warp) * RM_UNITS;
+  // operator of unit code x of stage st, and the fragments of the first one
+  auto oper = [&](int st, int x) {
+    return g0 + 4 * (p + 1) + (size_t)st * nst + ((x >> 7) ? c_rm.s[p + 1] : 0) + c_rm.s[(x & 127) - 1];
+  };
+  double an[RM_MT<NT>];
+  if (list[0]) rm_first<NT>(an, oper(0, list[0]), ((list[0] & 127) + 7) >> 3, lane);
+  // sources with Rz: lane (coefficient of 8, column of 4), both parts, the
+  // loads of RM_U steps in flight together
+  constexpr int RM_U = 4;
+  for (int q0 = warp; q0 < ncg * (NC / 4); q0 += RM_U * NW) {
+    double2 v[RM_U], R0[RM_U], R1[RM_U];
+    int at[RM_U];  // n << 16 | m << 8 | column, -1: none
+#pragma unroll
+    for (int u = 0; u < RM_U; u++) {
+      const int q = q0 + u * NW, c = (q % ncg) * 8 + (lane & 7), j = (q / ncg) * 4 + (lane >> 3);
+      at[u] = -1;
+      if (q >= ncg * (NC / 4) || c >= nc) continue;
+      at[u] = nm[c] << 8 | j;
+      const int m = nm[c] & 255;
+      const long long b = sb[j];
+      v[u] = b >= 0 ? __ldg(reinterpret_cast<const double2*>(src + b) + c) : make_double2(0.0, 0.0);
+      R0[u] = __ldg(reinterpret_cast<const double2*>(g0 + 4 * m));
+      R1[u] = __ldg(reinterpret_cast<const double2*>(g0 + 4 * m + 2));
+    }
+#pragma unroll
+    for (int u = 0; u < RM_U; u++) {
+      if (at[u] < 0) continue;
+      const int n = at[u] >> 16, m = at[u] >> 8 & 255, j = at[u] & 255;
+      const int cs = (j ^ (((n + m) & 3) << 2)) & (NC - 1);
+      X[(size_t)(n * n + m) * NC + cs] = R0[u].x * v[u].x + R0[u].y * v[u].y;
+      if (m > 0) X[(size_t)(n * n + n + m) * NC + cs] = R1[u].x * v[u].x + R1[u].y * v[u].y;
+    }
+  }
 #pragma unroll 1
   for (int st = 0; st < 3; st++) {
     __syncthreads();
-    const double* As = g0 + 4 * (p + 1) + (size_t)st * nst;
 #pragma unroll 1
     for (int u = 0; list[u]; u++) {
       const int r = list[u] & 127, part = list[u] >> 7;
-      const double* A = As + (part ? c_rm.s[p + 1] : 0) + c_rm.s[r - 1];
+      const double* A = oper(st, list[u]);
+      // the warp's next block, of this stage or the first of the next
+      const int xn = list[u + 1] ? list[u + 1] : (st < 2 ? list[0] : 0), mtn = ((xn & 127) + 7) >> 3;
+      const double* An = xn ? oper(list[u + 1] ? st : st + 1, xn) : A;
       const bool shift = st == 1;
       // Ry: degree n = r - 1 (re) or r (im, orders 1..n); shift: order m = p + 1 - r
       const int n = r - 1 + part, m = p + 1 - r;
       const int rb = n * n + (part ? n + 1 : 0), kb = shift ? 2 * m : n + part;
       switch ((r + 7) >> 3) {
-        case 1: rm_block<1, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
-        case 2: rm_block<2, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
-        case 3: rm_block<3, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
-        case 4: rm_block<4, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
-        case 5: if (NT < 4) rm_block<5, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
-        default: if (NT < 4) rm_block<6, NT>(X, A, r, shift, rb, m, part, kb, lane); break;
+        case 1: rm_block<1, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
+        case 2: rm_block<2, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
+        case 3: rm_block<3, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
+        case 4: rm_block<4, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
+        case 5: if constexpr (NT < 4) rm_block<5, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
+        default: if constexpr (NT < 4) rm_block<6, NT>(X, A, r, shift, rb, m, part, kb, lane, an, An, mtn); break;
       }
     }
   }
