@@ -83,8 +83,8 @@ __host__ __device__ inline long long l2t_ld(int P) { return (9LL * P + 3) & ~3LL
 // P2M of R (few) right-hand sides on the FP64 tensor cores (leaf_mma.cu), the
 // free-space passes (columns 4r + pass of C per box) or the image columns
 // (layout of launch_p2m_img); T = double ADDS to zeroed expansions, float
-// stores the normalised basis.  Returns false (nothing launched) when the
-// order is too high for its tiles.
+// (image columns only) stores the normalised basis.  Returns false (nothing
+// launched) when the order is too high for its tiles.
 template <class T, bool IMG>
 bool launch_p2m_mma(cudaStream_t st, int nleaf, const P2MArgs& a, int R, long long ubase, T* mpole);
 // L2T of R (few) right-hand sides likewise: free-space columns 4r + pass of C

@@ -371,7 +371,6 @@ bool launch_p2m_mma(cudaStream_t st, int nleaf, const P2MArgs& a, int R, long lo
   return true;
 }
 template bool launch_p2m_mma<double, false>(cudaStream_t, int, const P2MArgs&, int, long long, double*);
-template bool launch_p2m_mma<float, false>(cudaStream_t, int, const P2MArgs&, int, long long, float*);
 template bool launch_p2m_mma<double, true>(cudaStream_t, int, const P2MArgs&, int, long long, double*);
 template bool launch_p2m_mma<float, true>(cudaStream_t, int, const P2MArgs&, int, long long, float*);
 

@@ -54,14 +54,6 @@ double iprec_eps(int iprec) {
 // triangles + 2,003 targets, 0.052 against 0.232 on 1,000 triangles, 6.0
 // against 30.8 on 81,920 + 62,501, iprec 2, both layers with strain.
 constexpr int NEAR_LEAF_R = 4;
-// Mixed right-hand sides up to which P2M runs one by one on the FP64 tensor
-// cores (k_p2m_mma, float results) instead of unit multipoles and a product
-// whose 64 columns 4 R fill in part: the cost of the first grows with R, of
-// the second with the triangles only.  20,000 triangles at order 26: 1.13 /
-// 2.17 / 3.21 ms for R = 2 / 4 / 6 against 2.88; 1,000: 0.17 / 0.23 (R = 1 /
-// 4) against 0.24; at order 14 0.65 / 1.24 (R = 2 / 4) against 0.96.  Not
-// where the unit multipoles stay resident (stored near field, graphs).
-static int p2m_leaf_r(int p) { return p >= 20 ? 4 : 2; }
 
 int iprec_nbox(int iprec, int nsrc, int ntarg, bool iter) {
   int base;
@@ -2087,8 +2079,7 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
     if (mixed) {
       pa.wnorm = ops_->wnorm.get();  // multipoles in the normalised basis
       pick_engine(0, C);
-      if (R <= p2m_leaf_r(p_) && !resident_ && launch_p2m_mma<float, false>(st_, np2m_, pa, R, 0, mpole_f_.get())) {
-      } else if (!(p2m_unit_ && p2m_factored<float>(pa, R, mpole_f_.get(), false)))
+      if (!(p2m_unit_ && p2m_factored<float>(pa, R, mpole_f_.get(), false)))
         p2m_twostage<float>(pa, R, mpole_f_.get());
       rec(2);
       run_translations(m2m_, C, ops_->mats_f.get(), mpole_f_.get(), mpole_f_.get());
