@@ -1007,17 +1007,25 @@ void Plan::run_translations_tc(TransSched& S, int C, const float* src, float* ds
                   ops_->rot_tc_tiles.get(), D, C, b.pmax, src, dst, err);
 }
 
-// The engine of each FP32 translation stage for this pass: what the tuner
-// holds for the key (stage, order, leaf capacity, columns, kind), else the
-// CUDA cores.  The tensor cores were never the faster engine (orders 14 to
-// 30, 4 to 448 columns, each stage: 2.8 to 4.6 times slower, M2L of 64
-// columns at order 26 59.9 ms against 14.2), so no pass tries them: the first
-// passes of a key used to run them twice, and a pass captured into a graph
-// before the key was decided kept them (64 half-space right-hand sides on
-// 18,034 triangles: 42.1 ms a replay, 20.8 on the CUDA cores).
-void Plan::pick_engine(int kind, int C) {
-  for (int s = 0; s < 3; s++)
-    trans_cand_[s] = rot_tc_usable() ? tune_best(TuneKey{s, ops_->p, nbox_, C, 1, kind}, 1) : 1;
+// The engine of each FP32 translation stage for this pass: the tuner's pick
+// for the key (stage, order, leaf capacity, columns, kind); a pass being
+// captured into a graph takes the decided engine (or the tensor cores while
+// undecided) and reports nothing.  The engines round differently (6.6e-7 apart
+// on 81,920 triangles, one right-hand side; each 6e-7 from the FP64 pass), so
+// which one an undecided key runs is part of what a pass returns.  The CUDA
+// cores were faster at every key measured (orders 14 to 30, 4 to 448 columns:
+// M2L of 64 columns at order 26 14.2 ms against 59.9): a program that cannot
+// spare the first passes records the decision (efmm_tune_report, or
+// ELFMM3D_TUNE_FILE).
+void Plan::tune_begin(int kind, int C) {
+  trans_tuning_ = !capturing_ && rot_tc_usable();
+  for (int s = 0; s < 3; s++) {
+    trans_key_[s] = TuneKey{s, ops_->p, nbox_, C, 1, kind};
+    if (!rot_tc_usable())
+      trans_cand_[s] = 1;
+    else
+      trans_cand_[s] = capturing_ ? tune_best(trans_key_[s], 0) : tune_pick(trans_key_[s], 2);
+  }
 }
 
 void Plan::switch_precision(bool mixed) {
@@ -1040,6 +1048,13 @@ void Plan::switch_precision(bool mixed) {
     img_mp_.release();
     img_lc_.release();
   }
+}
+
+void Plan::tune_end() {
+  if (!trans_tuning_) return;
+  const float ms[3] = {timings.m2m, timings.m2l, timings.l2l};
+  for (int s = 0; s < 3; s++) tune_report(trans_key_[s], 2, trans_cand_[s], ms[s]);
+  trans_tuning_ = false;
 }
 
 template <class T>
@@ -2078,7 +2093,7 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
     pa.C = C; pa.rstride = 1; pa.tstride = 3 * (long long)R; pa.dstride = R;
     if (mixed) {
       pa.wnorm = ops_->wnorm.get();  // multipoles in the normalised basis
-      pick_engine(0, C);
+      tune_begin(0, C);
       if (!(p2m_unit_ && p2m_factored<float>(pa, R, mpole_f_.get(), false)))
         p2m_twostage<float>(pa, R, mpole_f_.get());
       rec(2);
@@ -2226,6 +2241,7 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   launches_ = (int)(launches_total() - launch0);
   product_collect();
   if (mixed && tc_take_error()) return IER_CUDA;  // a tensor-core product gave up waiting
+  if (mixed) tune_end();
   return IER_OK;
 }
 
@@ -2930,7 +2946,7 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
       float* mp = img_mp_f_.get();
       float* lc = img_lc_f_.get();
       pa.wnorm = ops_->wnorm.get();
-      pick_engine(1, Cv + Cu);
+      tune_begin(1, Cv + Cu);
       if (7 * R < 32)
         launch_p2m_img<float>(st_, np2m_, pa, R, (long long)(nb * Cv * D), mp);
       else if (!(p2m_unit_ && p2m_factored<float>(pa, R, mp, true)))
@@ -3054,6 +3070,7 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   launches_ = (int)(launches_total() - launch0);
   product_collect();
   if (mixed && tc_take_error()) return IER_CUDA;  // a tensor-core product gave up waiting
+  if (mixed) tune_end();
   return IER_OK;
 }
 

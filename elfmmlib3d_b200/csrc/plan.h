@@ -423,10 +423,14 @@ class Plan {
   bool rot_tc_usable() const;
   void cut_tc_tasks(TransSched& S, int C, bool one_launch);
   void run_translations_tc(TransSched& S, int C, const float* src, float* dst, bool one_launch);
-  // engine of the FP32 translations per stage (M2M, M2L, L2L): 0 tensor
-  // cores, 1 CUDA cores; chosen at the start of a mixed pass
-  int trans_cand_[3] = {1, 1, 1};
-  void pick_engine(int kind, int C);
+  // autotuned engine of the FP32 translations per stage (M2M, M2L, L2L):
+  // 0 tensor cores, 1 CUDA cores; chosen at the start of a mixed pass
+  // (tune_begin), reported with the stage times at its end (tune_end)
+  int trans_cand_[3] = {0, 0, 0};
+  TuneKey trans_key_[3];
+  bool trans_tuning_ = false;
+  void tune_begin(int kind, int C);
+  void tune_end();
   // A pass of the other precision than the last one releases the large
   // buffers only the last one's form uses (FP32 expansions, the FP32 copy
   // of the stored near field and the tensor-core intermediates; or the FP64

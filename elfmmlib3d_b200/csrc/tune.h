@@ -1,14 +1,14 @@
 // tune.h -- the autotuner (internal header; tune.cu).
 //
 // A knob is a choice between equivalent implementations of one stage of a
-// pass (the FP32 translations of the M2M, M2L and L2L stages on the tensor
-// cores or on the CUDA cores), made per key (knob, expansion order, leaf
-// capacity, expansion columns per box, precision, plan kind) from reported
-// times: pick goes through every candidate (twice each, the faster time kept)
-// and then keeps the fastest.  Decided keys are kept for the process and,
-// with ELFMM3D_TUNE_FILE set, in that file (read at the first use, a line
-// appended per decision) for later processes.  The passes themselves run
-// decided candidates only and explore none (Plan::pick_engine).
+// pass (for now: the FP32 translations of the M2M, M2L and L2L stages on
+// the tensor cores or on the CUDA cores).  The choice depends on the
+// problem's shape, so it is made per key (knob, expansion order, leaf
+// capacity, expansion columns per box, precision, plan kind) from timings of
+// the real passes: the first passes of a key run every candidate (twice
+// each, the faster time kept), later ones the fastest.  Decided keys are
+// kept for the process and, with ELFMM3D_TUNE_FILE set, in that file (read
+// at the first use, a line appended per decision) for later processes.
 #pragma once
 #include <string>
 #include <vector>
@@ -25,7 +25,8 @@ constexpr int TUNE_VISITS = 2;  // timed runs of each candidate before deciding
 
 // Candidate to run now for key k among ncand (0 .. ncand - 1).
 int tune_pick(const TuneKey& k, int ncand);
-// The decided candidate, or fallback while undecided.
+// The decided candidate, or fallback while undecided (no exploration: for
+// passes captured into a CUDA graph, which record no stage times).
 int tune_best(const TuneKey& k, int fallback);
 // A timed run of candidate cand for key k (stage milliseconds).
 void tune_report(const TuneKey& k, int ncand, int cand, float ms);

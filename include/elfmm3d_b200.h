@@ -548,12 +548,12 @@ int efmm_tc_bulk_selfcheck(int M, int N, int K, int bn, int fp64, unsigned seed,
 
 /* The autotuner (no counterpart in the reference, whose tuning is the fixed
  * iprec tables, src/elfmm3dtria.f:702-722): per key (knob, expansion order,
- * leaf capacity, expansion columns per box, precision, plan kind) the caller
- * runs the candidate that pick names (each TUNE_VISITS = 2 times, the faster
- * time kept, then the fastest).  Knobs 0, 1, 2: the FP32 translations of the
- * M2M, M2L, L2L stages on the tensor cores (candidate 0) or the CUDA cores
- * (1): a pass runs the decided candidate of its key, else the CUDA cores.
- * Decisions persist in the file named by ELFMM3D_TUNE_FILE when it is set.  pick
+ * leaf capacity, expansion columns per box, precision, plan kind) the first
+ * passes time every candidate implementation of the knob's stage
+ * (TUNE_VISITS = 2 runs each, the faster kept) and later passes run the
+ * fastest.  Knobs 0, 1, 2: the FP32 translations of the M2M, M2L, L2L
+ * stages on the tensor cores (candidate 0) or the CUDA cores (1).  Decisions
+ * persist in the file named by ELFMM3D_TUNE_FILE when it is set.  pick
  * returns the candidate to run; report records a timed run (ms); dump
  * writes "knob p nbox C prec kind decided ms..." lines into buf (len bytes)
  * and returns the full length. */

@@ -68,3 +68,41 @@ def test_few_right_hand_sides_as_in_a_batch(gpu, iprec, n, nrhs):
     gpu.load().efmm_tune_reset()
     for few, again, many in zip(*outs):
         assert rel(few, many) < 4.0 * rel(few, again)
+
+
+def _passes(gpu, P, n, R, count, seed=3, **more):
+    rng = np.random.default_rng(seed)
+    ssl, sdl = (_dev(a) for a in rng.normal(size=(2, R, n, 3)))
+    outs = []
+    for _ in range(count):
+        o = [_zeros(R, n, 3), _zeros(R, n, 3, 3), _zeros(R, 500, 3), _zeros(R, 500, 3, 3)]
+        P.evaluate_batch(1.3, 0.7, R, ssl, sdl, *o, precision=1, **more)
+        outs.append([t.cpu().numpy() for t in o])
+    return outs
+
+
+@pytest.mark.parametrize("nrhs", [1, 5])
+def test_first_passes_run_the_tuner_s_candidates(gpu, nrhs):
+    """The passes of an undecided key run the tensor-core translations twice,
+    then the CUDA-core ones twice, and a graph captured while undecided holds
+    the tensor cores.  The engine of a pass shows in its rounding: its outputs
+    are nearer to those of the same engine decided (they differ by the order of
+    the FP32 atomics, 1e-7) than to the other's (4e-7 and more)."""
+    n, L = 20480, gpu.load()
+    P = _plan(gpu, n, 2)
+    info = P.info()
+    key = (info["p"], info["nbox"], 4 * nrhs)
+    ref = []
+    for cand in (0, 1):
+        L.efmm_tune_reset()
+        _decide(L, *key, cand)
+        ref.append(_passes(gpu, P, n, nrhs, 1)[0])
+    engine = lambda o: int(np.argmin([sum(rel(a, b) for a, b in zip(o, r)) for r in ref]))  # noqa: E731
+    L.efmm_tune_reset()
+    assert [engine(o) for o in _passes(gpu, P, n, nrhs, 4)] == [0, 0, 1, 1]
+    L.efmm_tune_reset()
+    assert engine(_passes(gpu, P, n, nrhs, 1, graph=True)[0]) == 0
+    lines = [line.split() for line in gpu.tune_dump()]  # the pass before the capture reported, undecided
+    assert [(int(q[0]), int(q[3]), int(q[6])) for q in lines] == [(knob, 4 * nrhs, -1) for knob in range(3)]
+    P.close()
+    L.efmm_tune_reset()
