@@ -952,7 +952,8 @@ constexpr int NEAR_STREAM_R = 4;
 void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R,
                               int dostrain, const double* ssl, const double* sdl, int nsrc, int ntgt,
                               const long long* sbase, const int* sntri, const double* store) {
-  if (ntask <= 0 || R <= 0) return;
+  // without a layer the store is empty (K = 0) and there is nothing to add
+  if (ntask <= 0 || R <= 0 || !(a.dosl || a.dodl)) return;
   if (R > 64) throw CudaError{(int)cudaErrorInvalidValue};
   const int nlay = a.dosl + a.dodl, str = dostrain, K = nlay * 3 * (3 + 6 * dostrain), RB = (R + 15) / 16;
   const double* g0 = a.dosl ? ssl : sdl;
