@@ -115,6 +115,23 @@ EFMM_HD bool te_line(double len, double uA, double uB, double RA, double RB, dou
   return true;
 }
 
+// Offsets r from the vertices to X, distances R and their reciprocals, 0 at a
+// vertex itself (the ends' terms that diverge there are left out as the
+// edge's are).  Returns the signed distance from the plane, 0 for the
+// centroid (self) and at a vertex.
+EFMM_HD double te_vertices(const TriEdge& T, const double* X, bool self, double r[3][3], double R[3], double iR[3]) {
+  bool flat = self;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+#pragma unroll
+    for (int c = 0; c < 3; c++) r[k][c] = X[c] - T.v[3 * k + c];
+    R[k] = sqrt(te_dot(r[k], r[k]));
+    iR[k] = R[k] > 0.0 ? 1.0 / R[k] : 0.0;
+    flat = flat || R[k] == 0.0;
+  }
+  return flat ? 0.0 : te_dot(r[0], T.n);
+}
+
 // Response at X of one triangle: displacement u[3] and strain e[6] (if STR),
 // ADDED.  self: X is the triangle's centroid (principal value / finite part).
 // i2mu = 1 / 2 mu.
@@ -122,14 +139,7 @@ template <bool SL, bool DL>
 EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool str, double al, double i2mu, double* u,
                            double* e) {
   double r[3][3], R[3], iR[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) r[k][c] = X[c] - T.v[3 * k + c];
-    R[k] = sqrt(te_dot(r[k], r[k]));
-    iR[k] = 1.0 / R[k];
-  }
-  const double h = self ? 0.0 : te_dot(r[0], T.n);
+  const double h = te_vertices(T, X, self, r, R, iR);
   // signed solid angle (Van Oosterom and Strackee 1983), zero in the plane
   double om = 0.0;
   if (h != 0.0 && (SL || DL)) {
@@ -152,10 +162,12 @@ EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool st
     RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
     iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
     iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
-    const double uA = te_dot(rA, t), uB = uA - len;
+    // (exactly 0 at an end: the products round)
+    const bool end = RB == 0.0;
+    const double uA = end ? len : te_dot(rA, t), uB = end ? 0.0 : uA - len;
     double nu[3];
     te_cross(t, T.n, nu);
-    const double v = te_dot(rA, nu);
+    const double v = end ? 0.0 : te_dot(rA, nu);
     const double rho[3] = {v * nu[0] + h * T.n[0], v * nu[1] + h * T.n[1], v * nu[2] + h * T.n[2]};
     const double c2 = v * v + h * h;
     double L, K3, K5;
@@ -256,10 +268,11 @@ EFMM_HD bool te_edge(const TriEdge& T, int k, const double r[3][3], const double
   g.RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
   g.iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
   g.iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
-  g.uA = te_dot(rA, g.t);
-  g.uB = g.uA - T.len[k];
+  const bool end = g.RB == 0.0;
+  g.uA = end ? T.len[k] : te_dot(rA, g.t);
+  g.uB = end ? 0.0 : g.uA - T.len[k];
   te_cross(g.t, T.n, g.nu);
-  g.v = te_dot(rA, g.nu);
+  g.v = end ? 0.0 : te_dot(rA, g.nu);
   g.h = h;
 #pragma unroll
   for (int c = 0; c < 3; c++) g.rho[c] = g.v * g.nu[c] + h * T.n[c];
@@ -287,14 +300,7 @@ template <int LAYER, bool STR>
 EFMM_HD void tri_edge_blocks(const TriEdge& T, const double* X, bool self, double al, double i2mu, double* out) {
   constexpr int KB = STR ? 9 : 3;
   double r[3][3], R[3], iR[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-#pragma unroll
-    for (int c = 0; c < 3; c++) r[k][c] = X[c] - T.v[3 * k + c];
-    R[k] = sqrt(te_dot(r[k], r[k]));
-    iR[k] = 1.0 / R[k];
-  }
-  const double h = self ? 0.0 : te_dot(r[0], T.n);
+  const double h = te_vertices(T, X, self, r, R, iR);
   double om = 0.0;
   if (h != 0.0) {
     const double den = R[0] * R[1] * R[2] + te_dot(r[0], r[1]) * R[2] + te_dot(r[0], r[2]) * R[1] +
