@@ -85,14 +85,17 @@ EFMM_HD void te_sym(double* e, double f, const double* a, const double* b) {
 }
 
 // Edge integrals L, K3, K5 for ends at u_A, u_B = u_A - len along the edge
-// (target's coordinates), distances RA, RB, squared line distance c2.
-// Returns false when the target lies on the closed edge (its contribution is
-// left out, as in the reference, src/triahquad.f:1509).
-EFMM_HD bool te_line(double len, double uA, double uB, double RA, double RB, double iA, double iB, double c2,
+// (target's coordinates), distances RA, RB, squared line distance c2.  All
+// three diverge when the target lies on the closed edge and are left out
+// there (0, as in the reference, src/triahquad.f:1509); what the edge's ends
+// contribute stays: it carries the single layer's displacement, which is
+// continuous there.
+EFMM_HD void te_line(double len, double uA, double uB, double RA, double RB, double iA, double iB, double c2,
                      double& L, double& K3, double& K5) {
   const bool inside = uA > 0.0 && uB < 0.0;  // the foot of the target lies on the edge
   const double a = fabs(uA), b = fabs(uB), pA = RA + a, pB = RB + b, pp = pA * pB;
-  if (inside ? c2 == 0.0 : !(pp > 0.0)) return false;
+  L = K3 = K5 = 0.0;
+  if (inside ? c2 == 0.0 : !(pp > 0.0)) return;
   const double q = pA + pB, m = pp + c2;
   // inside: 1 / (c2 q); outside: 1 / (pA pB (pA pB + c2))
   const double inv = 1.0 / (inside ? c2 * q : pp * m);
@@ -112,7 +115,6 @@ EFMM_HD bool te_line(double len, double uA, double uB, double RA, double RB, dou
     K3 = d;
     K5 = d * (s - c2 * (1.0 / 3.0) * (s * s - gA * gB));
   }
-  return true;
 }
 
 // Offsets r from the vertices to X, distances R and their reciprocals, 0 at a
@@ -171,7 +173,7 @@ EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool st
     const double rho[3] = {v * nu[0] + h * T.n[0], v * nu[1] + h * T.n[1], v * nu[2] + h * T.n[2]};
     const double c2 = v * v + h * h;
     double L, K3, K5;
-    if (!te_line(len, uA, uB, RA, RB, iA, iB, c2, L, K3, K5)) continue;
+    te_line(len, uA, uB, RA, RB, iA, iB, c2, L, K3, K5);
     const double di = iA - iB;
     if (SL) {
       const double* s = T.s;
@@ -256,7 +258,7 @@ EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool st
 struct TeEdge {
   double t[3], nu[3], rho[3], v, h, RA, RB, uA, uB, iA, iB, L, K3, K5;
 };
-EFMM_HD bool te_edge(const TriEdge& T, int k, const double r[3][3], const double R[3], const double iR[3], double h,
+EFMM_HD void te_edge(const TriEdge& T, int k, const double r[3][3], const double R[3], const double iR[3], double h,
                      TeEdge& g) {
   double rA[3];
 #pragma unroll
@@ -276,7 +278,7 @@ EFMM_HD bool te_edge(const TriEdge& T, int k, const double r[3][3], const double
   g.h = h;
 #pragma unroll
   for (int c = 0; c < 3; c++) g.rho[c] = g.v * g.nu[c] + h * T.n[c];
-  return te_line(T.len[k], g.uA, g.uB, g.RA, g.RB, g.iA, g.iB, g.v * g.v + h * h, g.L, g.K3, g.K5);
+  te_line(T.len[k], g.uA, g.uB, g.RA, g.RB, g.iA, g.iB, g.v * g.v + h * h, g.L, g.K3, g.K5);
 }
 // e += f sym(e_k, b)
 EFMM_HD void te_sym_axis(double* e, int k, double f, const double* b) {
@@ -314,7 +316,7 @@ EFMM_HD void tri_edge_blocks(const TriEdge& T, const double* X, bool self, doubl
 #pragma unroll 1
   for (int k = 0; k < 3; k++) {
     TeEdge g;
-    if (!te_edge(T, k, r, R, iR, h, g)) continue;
+    te_edge(T, k, r, R, iR, h, g);
     const double di = g.iA - g.iB;
     if (LAYER == 1) {
       const double* t = g.t;

@@ -57,6 +57,13 @@ def test_vertices_are_finite(lib):
         pass
 
 
+def test_single_layer_displacement_is_its_limit_on_edges(lib):
+    """The displacement 1e-9 edge lengths off the plane is 1e-9 times its
+    gradient away, whose largest term there is log 1e9 = 21."""
+    for on, off in _on_mesh(lib, (0.0, 0.25, 0.5, 1.0 / 3.0, 0.9, 1.0)):
+        assert np.abs(on - off).max() < 1e-6 * np.abs(off).max()
+
+
 def _device_points(gpu, weights):
     """Targets on a mesh through the direct sum, a plan's near field alone
     (iprec 5: one box), one and several right-hand sides, analytic and stored,
@@ -95,3 +102,14 @@ def _device_points(gpu, weights):
 def test_device_at_vertices(gpu):
     for _, got, ref in _device_points(gpu, (0.0,)):
         assert np.isfinite(got).all() and rel(got, ref) < 1e-12
+
+
+@pytest.mark.gpu
+def test_device_on_edges(gpu):
+    """Off the vertices a point's distance from the edge rounds to 0 or not by
+    the order of the operations, and what diverges there with it: only the
+    displacement of the single layer is the same number on host and device."""
+    for layer, got, ref in _device_points(gpu, (0.0, 0.25, 0.5)):
+        assert np.isfinite(got).all()
+        if layer == 0:
+            assert rel(got[:, :3], ref[:, :3]) < 1e-12
