@@ -7,6 +7,14 @@
 
 namespace efmm {
 
+// Buffers that this thread has allocated, moved or freed and work lists that it
+// has uploaded (plan.cu h2d) so far.  A captured pass holds addresses and
+// sizes, so it outlives a plain pass only if the count stood still.
+inline long long& devbuf_changes() {
+  static thread_local long long n = 0;
+  return n;
+}
+
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -27,7 +35,10 @@ struct DevBuf {
     std::swap(cap, o.cap);
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p) {
+      cudaFree(p);
+      devbuf_changes()++;
+    }
     p = nullptr;
     n = cap = 0;
   }
@@ -38,6 +49,7 @@ struct DevBuf {
       size_t c = m ? m : 1;
       EFMM_CUDA_TRY(cudaMalloc((void**)&p, c * sizeof(T)));
       cap = c;
+      devbuf_changes()++;
     }
     n = m;
   }
@@ -56,6 +68,7 @@ struct DevBuf {
     p = q;
     cap = c;
     n = m;
+    devbuf_changes()++;
   }
   void zero(cudaStream_t st) {
     if (n) EFMM_CUDA_TRY(cudaMemsetAsync(p, 0, n * sizeof(T), st));

@@ -299,6 +299,7 @@ static std::vector<T> d2h(const DevBuf<T>& b, size_t n, cudaStream_t st) {
 template <class T>
 static void h2d(DevBuf<T>& b, const std::vector<T>& h, cudaStream_t st) {
   b.resize(h.size());
+  devbuf_changes()++;
   if (!h.empty()) EFMM_CUDA_TRY(cudaMemcpyAsync(b.get(), h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice, st));
 }
 
@@ -599,7 +600,7 @@ void Plan::build_worklists() {
   store_gen_++;
   ntc_key_ = -1;
   chunk_key_ = -1;
-  ntask_key_ = -1;
+  ntask_[0].key = ntask_[1].key = -1;
 
   mark("near");
   // far field
@@ -1125,8 +1126,10 @@ int Plan::store_alloc(int flags, double rlam, double rmu) {
   size_t freeb = 0, totb = 0;
   EFMM_CUDA_TRY(cudaMemGetInfo(&freeb, &totb));
   if ((double)tot * 8.0 > 0.9 * (double)freeb + (double)store_.cap * 8.0) return IER_ALLOC;
+  // a captured replay reads these blocks: it stays only if they will be the same
+  if (flags != store_flags_ || rlam != store_lam_ || rmu != store_mu_) graph_reset();
   store_.resize((size_t)tot);
-  h2d(near_base_, base, st_);
+  if (base != near_base_h_) h2d(near_base_, base, st_);
   near_base_h_ = base;
   store_K_ = K;
   store_flags_ = flags;
@@ -1287,6 +1290,7 @@ void Plan::near_tc(const NearArgs& na, int R, const double* g0, const double* g1
 
 int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d_sdl, double* d_u_src,
                    double* d_e_src, double* d_u_tgt, double* d_e_tgt, int mode, bool do_far) {
+  GraphGuard guard(*this);
   switch_precision(false);
   if (points_ && mode != 0) return IER_BADARG;  // particles: no stored near field
   int n = n_, nt = nt_;
@@ -1385,8 +1389,8 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     na.part_dl = dodl ? sdl_s_.get() : nullptr;
     launch_near_points(st_, na, nrm_s_.get(), rlam, rmu);
   } else if (mode == 0) {
-    build_near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
-    launch_near_leaf(st_, na, nntask_, ntask_.get());
+    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
+    launch_near_leaf(st_, na, w.n, w.t.get());
   } else {
     // stored operator rows carry displacement and (if any output wants it) strain
     NearArgs sa = na;
@@ -1399,8 +1403,8 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     NearArgs ra = na;  // outputs as requested by this call
     ra.dostrain_src = sa.dostrain_src;
     ra.dostrain_tgt = sa.dostrain_tgt;
-    build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
-    launch_near_replay_batch(st_, ra, nntask_, ntask_.get(), 1, sa.dostrain_src, ssl_s_.get(),
+    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+    launch_near_replay_batch(st_, ra, w.n, w.t.get(), 1, sa.dostrain_src, ssl_s_.get(),
                              sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   }
   EFMM_CUDA_TRY(cudaEventRecord(ev_[7], st_));
@@ -1537,6 +1541,7 @@ int Plan::evaluate_batch(double rlam, double rmu, int R, const double* d_ssl, co
                          int mode) {
   if (R < 1 || precision < 0 || precision > 1 || mode < 0 || mode > 2) return IER_BADARG;
   if (points_) return IER_BADARG;  // particles: the single-right-hand-side FP64 form only
+  GraphGuard guard(*this);
   switch_precision(precision == 1);
   MixedOrders orders(this, precision == 1);
   // the mixed form's geometry-only features stay resident for passes that
@@ -2200,20 +2205,20 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
     if (mixed && mode && near_tc_ready(na))
       near_tc(na, R, dosl ? ssl_s_.get() : sdl_s_.get(), sdl_s_.get(), n, nt);
     else if (mode == 0 && R <= NEAR_LEAF_R) {
-      build_near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
       for (int r = 0; r < R; r++) {
         launch_tri_edge_prep(st_, n, tri_s_.get(), ssl_s_.get(), sdl_s_.get(), dosl, dodl, tedge_.get(), R, r);
         NearArgs ra = na;
         ra.u_src += 3 * (size_t)n * r; ra.e_src += 6 * (size_t)n * r;
         ra.u_tgt += 3 * (size_t)nt * r; ra.e_tgt += 6 * (size_t)nt * r;
-        launch_near_leaf(st_, ra, nntask_, ntask_.get());
+        launch_near_leaf(st_, ra, w.n, w.t.get());
       }
     } else if (mode == 0) {
-      build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
-      launch_near_batch(st_, na, nntask_, ntask_.get(), R, (ds_src || ds_tgt) ? 1 : 0, ssl_s_.get(), sdl_s_.get(), n, nt);
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+      launch_near_batch(st_, na, w.n, w.t.get(), R, (ds_src || ds_tgt) ? 1 : 0, ssl_s_.get(), sdl_s_.get(), n, nt);
     } else {
-      build_near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
-      launch_near_replay_batch(st_, na, nntask_, ntask_.get(), R, (ds_src || ds_tgt) ? 1 : 0,
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+      launch_near_replay_batch(st_, na, w.n, w.t.get(), R, (ds_src || ds_tgt) ? 1 : 0,
                                ssl_s_.get(), sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
     }
   }
@@ -2247,6 +2252,7 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
 
 int Plan::evaluate_direct(double rlam, double rmu, const double* d_ssl, const double* d_sdl,
                           double* d_u_src, double* d_e_src, double* d_u_tgt, double* d_e_tgt, int nsub) {
+  GraphGuard guard(*this);
   int n = n_, nt = nsub > 0 ? 0 : nt_;
   int dosl = d_ssl != nullptr, dodl = d_sdl != nullptr;
   if (points_) {  // particles: the point-pair direct sum, user order
@@ -2623,9 +2629,10 @@ void Plan::build_chunks(int do_src, int do_tgt) {
 // CTAs on 148 SMs), but 512 at least (4 pairs per thread, below that staging
 // and the final sums dominate) and 16,384 at most; the items of at least W /
 // 2 pairs first, so the last ones to start are short.
-void Plan::build_near_tasks(int do_src, int do_tgt, int pts) {
-  const int key = do_src | (do_tgt << 1) | (pts << 2);
-  if (ntask_key_ == key) return;
+const Plan::NearTasks& Plan::near_tasks(int do_src, int do_tgt, int pts) {
+  NearTasks& out = ntask_[pts == NEAR_BATCH_PTS];
+  const int key = do_src | (do_tgt << 1);
+  if (out.key == key) return out;
   long long tot = 0;
   for (size_t i = 0; i < near_sc_h_.size(); i++)
     tot += (long long)((do_src ? near_sc_h_[i] : 0) + (do_tgt ? near_tc_h_[i] : 0)) * near_ntri_h_[i];
@@ -2644,14 +2651,15 @@ void Plan::build_near_tasks(int do_src, int do_tgt, int pts) {
       }
     }
   }
-  nntask_ = (int)(big.size() + small.size());
   big.insert(big.end(), small.begin(), small.end());
-  h2d(ntask_, big, st_);
-  if (nntask_) {
-    k_near_seek<<<(nntask_ + 127) / 128, 128, 0, st_>>>(nntask_, near_rstart_.get(), near_rng_.get(), ntask_.get());
+  out.n = (int)big.size();
+  h2d(out.t, big, st_);
+  if (out.n) {
+    k_near_seek<<<(out.n + 127) / 128, 128, 0, st_>>>(out.n, near_rstart_.get(), near_rng_.get(), out.t.get());
     count_launch();
   }
-  ntask_key_ = key;
+  out.key = key;
+  return out;
 }
 
 // Two-stage P2M of the image columns over waves of leaves (budget as in
@@ -2838,6 +2846,7 @@ int Plan::evaluate_image(double rlam, double rmu, int R, const double* d_ssl, co
   if (R < 1 || precision < 0 || precision > 1 || mode < 0 || mode > 2) return IER_BADARG;
   if (!mindlin_ || rmu <= 0 || rlam + 2 * rmu <= 0) return IER_BADARG;
   if (points_ && (precision != 0 || 7 * R >= 32)) return IER_BADARG;  // particles: FP64, at most 4 right-hand sides
+  GraphGuard guard(*this);
   switch_precision(precision == 1);
   resident_ = precision == 1 && (mode != 0 || graph_pass_);
   const int nt = nt_;
@@ -3048,8 +3057,8 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   na.do_src = 0; na.do_tgt = 1;
   na.rlam = rlam; na.rmu = rmu;
   na.u_src = nullptr; na.e_src = nullptr; na.u_tgt = ut_s_.get(); na.e_tgt = et_s_.get();
-  build_near_tasks(0, 1, NEAR_BATCH_PTS);
-  launch_near_replay_batch(st_, na, nntask_, ntask_.get(), R, dstr, ssl_s_.get(), sdl_s_.get(),
+  const NearTasks& w = near_tasks(0, 1, NEAR_BATCH_PTS);
+  launch_near_replay_batch(st_, na, w.n, w.t.get(), R, dstr, ssl_s_.get(), sdl_s_.get(),
                            n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   rec(7);
   k_scatter_out<<<dim3((nt + 255) / 256, R), 256, 0, st_>>>(nt, tr_.izt.get(), ut_s_.get(), et_s_.get(), d_u_tgt,

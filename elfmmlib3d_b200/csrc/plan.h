@@ -233,6 +233,9 @@ class Plan {
   // identical pass and launches the graph; later calls with the same key
   // only launch it.  Batch: mode 0 or 2 (the store made by an earlier mode-1
   // call); image: mode 2.  New data must be written into the same buffers.
+  // Other passes may run in between: one that moves a buffer or refills a
+  // work list which the captured pass holds drops it, and the next call
+  // captures again.
   int evaluate_batch_graph(double rlam, double rmu, int R, const double* d_ssl, const double* d_sdl,
                            double* d_u_src, double* d_e_src, double* d_u_tgt, double* d_e_tgt, int precision,
                            int mode);
@@ -279,7 +282,11 @@ class Plan {
   void ensure_mats_f();
   int build_image_sched();
   void build_chunks(int do_src, int do_tgt);
-  void build_near_tasks(int do_src, int do_tgt, int pts);
+  struct NearTasks {  // work items of the near field
+    DevBuf<NearTask> t;
+    int n = 0, key = -1;
+  };
+  const NearTasks& near_tasks(int do_src, int do_tgt, int pts);
   bool mindlin_ = false, img_sched_ = false;
   bool forest_on_ = false;
   // keep the geometry-only features of the two-stage P2M / L2T between
@@ -321,13 +328,22 @@ class Plan {
   long long graph_launches_ = 0;
   void rec(int i);
   void graph_reset();
+  // Around a pass: drops the captured one if a buffer or list of this plan
+  // that it may hold has moved or been filled anew.
+  struct GraphGuard {
+    Plan& p;
+    const long long at;
+    explicit GraphGuard(Plan& q) : p(q), at(devbuf_changes()) {}
+    ~GraphGuard() {
+      if (devbuf_changes() != at) p.graph_reset();
+    }
+  };
   int run_graph(const std::vector<double>& key, const std::function<int()>& pass);
   DevBuf<float> img_mp_f_, img_lc_f_;
   DevBuf<float> mpole_f_, local_f_;
   DevBuf<int> chunk_leaf_, chunk_e0_;  // (near leaf, first point) per batched near-field CTA
   int nchunk_ = 0, chunk_key_ = -1;
-  DevBuf<NearTask> ntask_;  // work items of the one-right-hand-side near field
-  int nntask_ = 0, ntask_key_ = -1;
+  NearTasks ntask_[2];  // of NEAR_TASK_PTS and of NEAR_BATCH_PTS points
   std::vector<int> l2t_sc_h_, l2t_tc_h_;  // per L2T leaf
   std::vector<int> l2t_h_;                // L2T leaves
   DevBuf<double> l2t_scratch_;            // functionals + sums of one wave of leaves

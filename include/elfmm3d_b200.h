@@ -391,7 +391,9 @@ int efmm_tc_gemm_selfcheck_tile(int M, int N, int K, int bn, int aligned, unsign
  * mode-1 call); image: the stored near field of an earlier mode-1 call.
  * nrhs <= 64 (one pass per call; else IER 16).
  * The first call should not run while another capture on the plan's stream
- * is in progress.  A new geometry drops the graph. */
+ * is in progress.  A new geometry drops the graph, and so does another call on
+ * the plan (plain, or of other parameters) that moves a buffer or refills a
+ * work list; the next graph call then captures again. */
 int efmm_plan_evaluate_batch_graph(efmm_plan *plan, double rlam, double rmu, int nrhs, const double *ssl,
                                    const double *sdl, double *u_src, double *e_src, double *u_tgt,
                                    double *e_tgt, int precision, int mode);
