@@ -48,8 +48,24 @@ double hs_quad_eps(int iprec) {
   return e > 0.0 ? fmin(1e-6, 0.1 * e) : 1e-16;
 }
 
-// The sub-triangle of v0 along a path of halvings (2 bits each, the first in
-// the highest bits).
+// Child k of the sub-triangle a, b, c (halved edges), in its place.
+__device__ __forceinline__ void hs_child(int k, double a[3], double b[3], double c[3]) {
+  double ab[3], bc[3], ca[3];
+  for (int d = 0; d < 3; d++) {
+    ab[d] = 0.5 * (a[d] + b[d]);
+    bc[d] = 0.5 * (b[d] + c[d]);
+    ca[d] = 0.5 * (c[d] + a[d]);
+  }
+  for (int d = 0; d < 3; d++) {
+    if (k == 0) { b[d] = ab[d]; c[d] = ca[d]; }
+    else if (k == 1) { a[d] = ab[d]; c[d] = bc[d]; }
+    else if (k == 2) { a[d] = ca[d]; b[d] = bc[d]; }
+    else { a[d] = ab[d]; b[d] = bc[d]; c[d] = ca[d]; }
+  }
+}
+
+// The sub-triangle of v0 along a path of at most HS_ADAPT_DEPTH halvings (2
+// bits each, the first in the highest bits).
 __device__ __forceinline__ void hs_descend(const double* v0, unsigned int cd, int depth, double a[3], double b[3],
                                            double c[3]) {
   for (int d = 0; d < 3; d++) {
@@ -57,21 +73,7 @@ __device__ __forceinline__ void hs_descend(const double* v0, unsigned int cd, in
     b[d] = v0[3 + d];
     c[d] = v0[6 + d];
   }
-  for (int l = depth - 1; l >= 0; l--) {
-    const int k = (cd >> (2 * l)) & 3;
-    double ab[3], bc[3], ca[3];
-    for (int d = 0; d < 3; d++) {
-      ab[d] = 0.5 * (a[d] + b[d]);
-      bc[d] = 0.5 * (b[d] + c[d]);
-      ca[d] = 0.5 * (c[d] + a[d]);
-    }
-    for (int d = 0; d < 3; d++) {
-      if (k == 0) { b[d] = ab[d]; c[d] = ca[d]; }
-      else if (k == 1) { a[d] = ab[d]; c[d] = bc[d]; }
-      else if (k == 2) { a[d] = ca[d]; b[d] = bc[d]; }
-      else { a[d] = ab[d]; b[d] = bc[d]; c[d] = ca[d]; }
-    }
-  }
+  for (int l = depth - 1; l >= 0; l--) hs_child((cd >> (2 * l)) & 3, a, b, c);
 }
 
 __device__ __forceinline__ double hs_area(const double* a, const double* b, const double* c) {
@@ -384,8 +386,10 @@ __device__ __noinline__ void hs_adapt_blk(const double* v0, const double* nrm, c
     --top;
     const unsigned int cd = code[top];
     const int depth = dep[top];
-    double I[27], S[27];
-    // pass 0 the rule on the sub-triangle, pass 1 on its four children
+    double I[27], S[27], sa[3], sb[3], sc[3];
+    hs_descend(v0, cd, depth, sa, sb, sc);
+    // pass 0 the rule on the sub-triangle, pass 1 on its four children (whose
+    // paths have one digit more than cd holds at the last depth)
 #pragma unroll 1
     for (int pass = 0; pass < 2; pass++) {
       M m;
@@ -393,7 +397,12 @@ __device__ __noinline__ void hs_adapt_blk(const double* v0, const double* nrm, c
 #pragma unroll 1
       for (int k = 0; k < (pass ? 4 : 1); k++) {
         double a[3], b[3], c[3];
-        hs_descend(v0, pass ? (cd << 2) | (unsigned int)k : cd, depth + pass, a, b, c);
+        for (int d = 0; d < 3; d++) {
+          a[d] = sa[d];
+          b[d] = sb[d];
+          c[d] = sc[d];
+        }
+        if (pass) hs_child(k, a, b, c);
         hs_rule(a, b, c, X, m);
       }
       assemble(m, S);
