@@ -4,6 +4,8 @@
 // ITER variant src/elfmm3dtria_iter_1.f:1240-1419) sums, for each evaluation
 // point, the exact single/double layer potential of every triangle in the
 // source boxes paired with the point's leaf box.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "common.cuh"
@@ -142,27 +144,37 @@ k_near_leaf(const NearArgs a, const NearTask* __restrict__ tasks) {
   }
 }
 
-// All-pairs direct sum (el3dtriadirecttarg, src/elfmm3dtria.f:1483): one
-// thread per evaluation point, all triangles streamed through shared memory;
-// gridDim.y CTAs share the triangles of a block of points (outputs zeroed by
-// the launcher and added to).  Points [0, nsrc) are the centroids (self pair
-// when the indices match), [nsrc, nsrc + ntgt) the targets.
+// All-pairs direct sum (el3dtriadirecttarg, src/elfmm3dtria.f:1483): a CTA
+// holds ND_PTS points, its 16 slices of threads and the CTAs of a cluster share
+// the triangles, streamed through shared memory.  The parts are added in a
+// fixed order through the cluster's shared memory, so that a call repeats bit
+// for bit.  Points [0, nsrc) are the centroids (self pair when the indices
+// match), [nsrc, nsrc + ntgt) the targets.  Points per CTA 4 / 8 / 16 / 32 /
+// 128: 3.33 / 3.17 / 3.22 / 3.63 / 3.73 ms on 5,120 triangles + 1,000 targets,
+// 75 / 73 / 75 / 75 / 82 on 20,480 + 20,000, .104 / .096 / .119 / .122 / .270 on
+// 317 + 41 (parts of the triangles added atomically, 128 points: 3.40, 74.7,
+// .152).
+constexpr int ND_PTS = 8;
 template <bool SL, bool DL>
 __global__ void __launch_bounds__(NL_THREADS, NL_MINB)
 k_direct_all(int ntri, const TriEdge* __restrict__ rec, int nsrc, const double* __restrict__ src_pts, int ntgt,
              const double* __restrict__ tgt_pts, int dostrain_src, int dostrain_tgt, double rlam, double rmu,
              double* __restrict__ u_src, double* __restrict__ e_src, double* __restrict__ u_tgt,
              double* __restrict__ e_tgt) {
-  __shared__ __align__(16) double tile[NL_TILE * NL_STRIDE];
-  const int tid = threadIdx.x, ep = blockIdx.x * NL_THREADS + tid;
+  constexpr int P = ND_PTS, S = NL_THREADS / P;
+  constexpr int NT = NL_TILE * NL_STRIDE > 9 * NL_THREADS ? NL_TILE * NL_STRIDE : 9 * NL_THREADS;
+  __shared__ __align__(16) double tile[NT];  // the triangles, then the threads' sums
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int tid = threadIdx.x, sl = tid / P, ep = blockIdx.x * P + tid % P;
   const bool on = ep < nsrc + ntgt, is_src = ep < nsrc;
   const int pidx = is_src ? ep : ep - nsrc;
   const bool str = is_src ? dostrain_src : dostrain_tgt;
   const double al = (rlam + rmu) / (rlam + 2.0 * rmu), i2mu = 0.5 / rmu;
   double X[3] = {0, 0, 0};
   if (on) {
-    const double* P = (is_src ? src_pts : tgt_pts) + 3 * (size_t)pidx;
-    X[0] = P[0]; X[1] = P[1]; X[2] = P[2];
+    const double* Q = (is_src ? src_pts : tgt_pts) + 3 * (size_t)pidx;
+    X[0] = Q[0]; X[1] = Q[1]; X[2] = Q[2];
   }
   const int lo = (int)((long long)ntri * blockIdx.y / gridDim.y);
   const int hi = (int)((long long)ntri * (blockIdx.y + 1) / gridDim.y);
@@ -175,17 +187,34 @@ k_direct_all(int ntri, const TriEdge* __restrict__ rec, int nsrc, const double* 
       reinterpret_cast<double2*>(tile + (q / 16) * NL_STRIDE)[q % 16] = src[q];
     __syncthreads();
     if (on)
-      for (int t = 0; t < m; t++) {
+      for (int t = sl; t < m; t += S) {
         const TriEdge& T = *reinterpret_cast<const TriEdge*>(tile + t * NL_STRIDE);
         tri_edge_pair<SL, DL>(T, X, is_src && k0 + t == pidx, str, al, i2mu, u, ee);
       }
   }
-  if (!on) return;
-  double* U = (is_src ? u_src : u_tgt) + 3 * (size_t)pidx;
-  double* E = (is_src ? e_src : e_tgt) + 6 * (size_t)pidx;
-  for (int c = 0; c < 3; c++) atomicAdd(U + c, u[c]);
-  if (str)
-    for (int c = 0; c < 6; c++) atomicAdd(E + c, ee[c]);
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < 3; c++) tile[c * NL_THREADS + tid] = u[c];
+#pragma unroll
+  for (int c = 0; c < 6; c++) tile[(3 + c) * NL_THREADS + tid] = ee[c];
+  cl.sync();
+  // (gridDim.y CTAs are the cluster; its first one adds)
+  if (blockIdx.y == 0)
+    for (int q = tid; q < 9 * P; q += NL_THREADS) {
+      const int c = q / P, e = blockIdx.x * P + q % P;
+      if (e >= nsrc + ntgt) continue;
+      const bool src = e < nsrc;
+      if (c >= 3 && !(src ? dostrain_src : dostrain_tgt)) continue;
+      double v = 0.0;
+      for (int y = 0; y < (int)gridDim.y; y++) {
+        const double* part = cl.map_shared_rank(tile, y) + c * NL_THREADS + q % P;
+        for (int w = 0; w < S; w++) v += part[w * P];
+      }
+      const size_t i = src ? e : e - nsrc;
+      if (c < 3) (src ? u_src : u_tgt)[3 * i + c] = v;
+      else (src ? e_src : e_tgt)[6 * i + c - 3] = v;
+    }
+  cl.sync();  // the parts stay until they are read
 }
 
 // ITER mode, first call: compute and store the unit-density response blocks
@@ -497,7 +526,11 @@ k_near_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R, int K,
 // inner loop unrolled.  Same tiling as k_near_batch (work items of 8 points, 16
 // triangles per tile, 9 x RB outputs per thread).  Items instead of whole
 // lists: the image replay of 64 right-hand sides on 18,034 triangles, where few
-// points have near triangles, 10.5 -> 4.1 ms.
+// points have near triangles, 10.5 -> 4.1 ms.  The next tile's triangles are
+// looked up while this one's are read, so that a tile costs two barriers, and
+// the densities are read before the store: 5 right-hand sides, near field alone
+// of 5,120 triangles + 1,000 targets 12.5 ms (three barriers 21, the store
+// first 23).
 template <int RB, int NLAY, int STR>
 __global__ void __launch_bounds__(NB_THREADS)
 k_near_replay_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R,
@@ -508,7 +541,7 @@ k_near_replay_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R,
   extern __shared__ __align__(16) double rb_sm[];
   double* Bk = rb_sm;                     // [NB_PTS][NB_TRI][K]
   double* Sg = Bk + NB_PTS * NB_TRI * K;  // [NB_TRI][NJ][RW]
-  __shared__ int tidx[NB_TRI];
+  __shared__ int tidx[2][NB_TRI];  // this tile's triangles and the next one's
   const NearTask w = tasks[blockIdx.x];
   const int leaf = a.leaves[w.li];
   const int s0 = a.box_src_start[leaf], sn = a.do_src ? a.box_src_count[leaf] : 0, t0 = a.box_tgt_start[leaf];
@@ -522,13 +555,12 @@ k_near_replay_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R,
 #pragma unroll
     for (int k = 0; k < RB; k++) acc[c][k] = 0.0;
   int b = w.r0, k = w.k0;  // range and triangle of the range to stage next
-  for (int pos = 0; pos < w.cnt; pos += NB_TRI) {
+  auto stage = [&](int pos, int* to) {  // the triangles of the tile at pos, across ranges
     const int cnt = min(NB_TRI, w.cnt - pos);
-    __syncthreads();
-    for (int fill = 0; fill < cnt;) {  // the tile's triangles, across ranges
+    for (int fill = 0; fill < cnt;) {
       const int2 rg = a.rng[b];
       const int m = min(cnt - fill, rg.y - k);
-      if (tid < m) tidx[fill + tid] = rg.x + k + tid;
+      if (tid < m) to[fill + tid] = rg.x + k + tid;
       fill += m;
       k += m;
       if (k >= rg.y) {
@@ -536,20 +568,25 @@ k_near_replay_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R,
         k = 0;
       }
     }
+  };
+  stage(0, tidx[0]);
+  for (int pos = 0; pos < w.cnt; pos += NB_TRI) {
+    const int cnt = min(NB_TRI, w.cnt - pos), cur = (pos / NB_TRI) & 1;
+    __syncthreads();
+    for (int q = tid; q < NB_TRI * NJ * RW; q += NB_THREADS) {
+      const int t = q / (NJ * RW), j = (q / RW) % NJ, r = q % RW;
+      const double* sg = (NLAY == 2 && j >= 3) ? sg1 : sg0;
+      double v = 0.0;
+      if (t < cnt && r < R) v = sg[((size_t)tidx[cur][t] * 3 + (j % 3)) * R + r];
+      Sg[q] = v;
+    }
     for (int q = tid; q < NB_PTS * NB_TRI * K; q += NB_THREADS) {
       const int pt = q / (NB_TRI * K), rem = q % (NB_TRI * K);
       double v = 0.0;
       if (pt < w.ne && rem < cnt * K) v = __ldcs(src + ((size_t)pt * nt + pos) * K + rem);
       Bk[q] = v;
     }
-    __syncthreads();
-    for (int q = tid; q < NB_TRI * NJ * RW; q += NB_THREADS) {
-      const int t = q / (NJ * RW), j = (q / RW) % NJ, r = q % RW;
-      const double* sg = (NLAY == 2 && j >= 3) ? sg1 : sg0;
-      double v = 0.0;
-      if (t < cnt && r < R) v = sg[((size_t)tidx[t] * 3 + (j % 3)) * R + r];
-      Sg[q] = v;
-    }
+    if (pos + NB_TRI < w.cnt) stage(pos + NB_TRI, tidx[cur ^ 1]);
     __syncthreads();
     const double* Bp = Bk + pq * NB_TRI * K;
 #pragma unroll 2
@@ -1004,21 +1041,25 @@ void launch_direct_all(cudaStream_t st, int ntri, const TriEdge* rec, int nsrc, 
                        double rmu, double* u_src, double* e_src, double* u_tgt, double* e_tgt) {
   const int nep = nsrc + ntgt;
   if (nep <= 0) return;
-  if (nsrc > 0) {
-    EFMM_CUDA_TRY(cudaMemsetAsync(u_src, 0, 24 * (size_t)nsrc, st));
-    EFMM_CUDA_TRY(cudaMemsetAsync(e_src, 0, 48 * (size_t)nsrc, st));
-  }
-  if (ntgt > 0) {
-    EFMM_CUDA_TRY(cudaMemsetAsync(u_tgt, 0, 24 * (size_t)ntgt, st));
-    EFMM_CUDA_TRY(cudaMemsetAsync(e_tgt, 0, 48 * (size_t)ntgt, st));
-  }
-  // parts of the triangles so that few points still cover the chip about
-  // three times (3 CTAs per SM), but no part of fewer than about 16
-  const int nb = (nep + NL_THREADS - 1) / NL_THREADS, want = (3 * 3 * 148 + nb - 1) / nb;
-  const dim3 grid(nb, std::max(1, std::min({want, (ntri + 15) / 16, 64})));
+  // up to 8 CTAs (a cluster) share the triangles of a block of points so that
+  // few points still cover the chip about three times (3 CTAs per SM), but no
+  // part of fewer than about 16
+  const int nb = (nep + ND_PTS - 1) / ND_PTS;
+  const int parts = std::max(1, std::min({(3 * 3 * 148 + nb - 1) / nb, (ntri + 15) / 16, 8}));
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = 1;
+  at.val.clusterDim.y = parts;
+  at.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nb, parts);
+  cfg.blockDim = dim3(NL_THREADS);
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
   auto go = [&](auto kern) {
-    kern<<<grid, NL_THREADS, 0, st>>>(ntri, rec, nsrc, src_pts, ntgt, tgt_pts, dostrain_src, dostrain_tgt, rlam, rmu,
-                                      u_src, e_src, u_tgt, e_tgt);
+    EFMM_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, ntri, rec, nsrc, src_pts, ntgt, tgt_pts, dostrain_src,
+                                     dostrain_tgt, rlam, rmu, u_src, e_src, u_tgt, e_tgt));
   };
   if (dosl && dodl)
     go(k_direct_all<true, true>);

@@ -1389,7 +1389,7 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     na.part_dl = dodl ? sdl_s_.get() : nullptr;
     launch_near_points(st_, na, nrm_s_.get(), rlam, rmu);
   } else if (mode == 0) {
-    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
+    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS, far_ && do_far);
     launch_near_leaf(st_, na, w.n, w.t.get());
   } else {
     // stored operator rows carry displacement and (if any output wants it) strain
@@ -1403,7 +1403,7 @@ int Plan::evaluate(double rlam, double rmu, const double* d_ssl, const double* d
     NearArgs ra = na;  // outputs as requested by this call
     ra.dostrain_src = sa.dostrain_src;
     ra.dostrain_tgt = sa.dostrain_tgt;
-    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+    const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS, far_ && do_far);
     launch_near_replay_batch(st_, ra, w.n, w.t.get(), 1, sa.dostrain_src, ssl_s_.get(),
                              sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   }
@@ -2205,7 +2205,7 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
     if (mixed && mode && near_tc_ready(na))
       near_tc(na, R, dosl ? ssl_s_.get() : sdl_s_.get(), sdl_s_.get(), n, nt);
     else if (mode == 0 && R <= NEAR_LEAF_R) {
-      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS);
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_TASK_PTS, far_);
       for (int r = 0; r < R; r++) {
         launch_tri_edge_prep(st_, n, tri_s_.get(), ssl_s_.get(), sdl_s_.get(), dosl, dodl, tedge_.get(), R, r);
         NearArgs ra = na;
@@ -2214,10 +2214,10 @@ int Plan::batch_pass(double rlam, double rmu, int R, const double* d_ssl, const 
         launch_near_leaf(st_, ra, w.n, w.t.get());
       }
     } else if (mode == 0) {
-      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS, far_);
       launch_near_batch(st_, na, w.n, w.t.get(), R, (ds_src || ds_tgt) ? 1 : 0, ssl_s_.get(), sdl_s_.get(), n, nt);
     } else {
-      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS);
+      const NearTasks& w = near_tasks(do_src, do_tgt, NEAR_BATCH_PTS, far_);
       launch_near_replay_batch(st_, na, w.n, w.t.get(), R, (ds_src || ds_tgt) ? 1 : 0,
                                ssl_s_.get(), sdl_s_.get(), n, nt, near_base_.get(), near_ntri_.get(), store_.get());
     }
@@ -2623,26 +2623,37 @@ void Plan::build_chunks(int do_src, int do_tgt) {
   chunk_key_ = key;
 }
 
-// Work items of the analytic near field, at most pts evaluation points each
-// (NEAR_TASK_PTS: one right-hand side, NEAR_BATCH_PTS: several).  An item
-// holds at most W pairs: an eighth of a resident slot's share of all pairs (3
-// CTAs on 148 SMs), but 512 at least (4 pairs per thread, below that staging
-// and the final sums dominate) and 16,384 at most; the items of at least W /
-// 2 pairs first, so the last ones to start are short.
-const Plan::NearTasks& Plan::near_tasks(int do_src, int do_tgt, int pts) {
+// Work items of the near field, at most pts evaluation points each
+// (NEAR_TASK_PTS: one right-hand side, NEAR_BATCH_PTS: several or stored).
+// Beside a far field (far) a leaf's triangles are cut so that an item holds
+// about W pairs: an eighth of a resident slot's share of all pairs (3 CTAs on
+// 148 SMs), but 512 at least (4 pairs per thread, below that staging and the
+// final sums dominate; no part below 16 triangles) and 16,384 at most, or a
+// millionth of all pairs if that is more; the items of at least W / 2 pairs
+// first, so the last ones to start are short.  Parts are added atomically, in
+// any order.  Without a far field, whose sums have no fixed order either, a
+// pass repeats bit for bit: an item holds all triangles of its points, and of
+// the NEAR_TASK_PTS ones, whose threads share a point's triangles, as many
+// fewer points (a power of two, 4 at least) as give every SM three items.
+const Plan::NearTasks& Plan::near_tasks(int do_src, int do_tgt, int pts, bool far) {
   NearTasks& out = ntask_[pts == NEAR_BATCH_PTS];
-  const int key = do_src | (do_tgt << 1);
+  const int key = do_src | (do_tgt << 1) | (far << 2);
   if (out.key == key) return out;
-  long long tot = 0;
-  for (size_t i = 0; i < near_sc_h_.size(); i++)
-    tot += (long long)((do_src ? near_sc_h_[i] : 0) + (do_tgt ? near_tc_h_[i] : 0)) * near_ntri_h_[i];
-  const long long W = std::min<long long>(16384, std::max<long long>(512, tot / (8 * 3 * 148)));
+  long long tot = 0, npts = 0;
+  for (size_t i = 0; i < near_sc_h_.size(); i++) {
+    const int nep = (do_src ? near_sc_h_[i] : 0) + (do_tgt ? near_tc_h_[i] : 0);
+    npts += nep;
+    tot += (long long)nep * near_ntri_h_[i];
+  }
+  const long long W = std::min<long long>(std::max<long long>(16384, tot >> 20), std::max<long long>(512, tot / (8 * 3 * 148)));
+  if (!far && pts == NEAR_TASK_PTS)
+    while (pts > 4 && npts < 3LL * 148 * pts) pts /= 2;
   std::vector<NearTask> big, small;
   for (size_t i = 0; i < near_sc_h_.size(); i++) {
     const int nep = (do_src ? near_sc_h_[i] : 0) + (do_tgt ? near_tc_h_[i] : 0), nt = near_ntri_h_[i];
     if (nep == 0 || nt == 0) continue;
     const int nch = (nep + pts - 1) / pts, cs = (nep + nch - 1) / nch;
-    const int parts = (int)std::min<long long>((nt + 15) / 16, ((long long)cs * nt + W - 1) / W);
+    const int parts = far ? (int)std::min<long long>((nt + 15) / 16, ((long long)cs * nt + W - 1) / W) : 1;
     for (int q = 0; q < parts; q++) {
       const int cnt = (int)((long long)nt * (q + 1) / parts - (long long)nt * q / parts);
       for (int e0 = 0; e0 < nep; e0 += cs) {
@@ -3057,7 +3068,7 @@ int Plan::image_pass(double rlam, double rmu, int R, const double* d_ssl, const 
   na.do_src = 0; na.do_tgt = 1;
   na.rlam = rlam; na.rmu = rmu;
   na.u_src = nullptr; na.e_src = nullptr; na.u_tgt = ut_s_.get(); na.e_tgt = et_s_.get();
-  const NearTasks& w = near_tasks(0, 1, NEAR_BATCH_PTS);
+  const NearTasks& w = near_tasks(0, 1, NEAR_BATCH_PTS, far_);
   launch_near_replay_batch(st_, na, w.n, w.t.get(), R, dstr, ssl_s_.get(), sdl_s_.get(),
                            n, nt, near_base_.get(), near_ntri_.get(), store_.get());
   rec(7);

@@ -286,7 +286,7 @@ class Plan {
     DevBuf<NearTask> t;
     int n = 0, key = -1;
   };
-  const NearTasks& near_tasks(int do_src, int do_tgt, int pts);
+  const NearTasks& near_tasks(int do_src, int do_tgt, int pts, bool far);
   bool mindlin_ = false, img_sched_ = false;
   bool forest_on_ = false;
   // keep the geometry-only features of the two-stage P2M / L2T between
