@@ -673,6 +673,7 @@ def run_batch(args, rank, world, local_rank):
     value = replica_value(evals * args.steps, t_max, world)
     info = P.info()
     fl = P.flops_per_column()
+    fl.update({k: v / (4 * R) for k, v in P.translation_flops(R, precision=1).items()})  # the timed mixed form's
     setup = P.setup_timings()
     tim = {k: float(np.mean([s_[k] for s_ in stage])) for k in stage[0]}
     u_mixed, e_mixed = u.clone(), e.clone()

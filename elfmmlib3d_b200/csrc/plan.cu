@@ -1436,21 +1436,25 @@ void Plan::flops_per_column(double* f) const {
   const long long nodes = 12LL * n_;
   f[0] = 2.0 * D * 4.0 * (double)nodes;  // rows x (charge + 3 dipole) per node
   const TransSched* S[3] = {&m2m_, &m2l_, &l2l_};
-  // flops of the form that runs: factored (two rotations and the shift along
-  // z, each sum_{j=1}^{p+1} (2j)^2 multiply-adds) or dense (dim^2)
-  const bool fact = factored_ && 2.0 * D * rot_cols_per_cta((int)D, 4) * 4 <= 227.0 * 1024;
   for (int k = 0; k < 3; k++)
-    for (const TransSeg& g : S[k]->segs) {
-      if (fact) {
-        const double q = ops_->descs[g.group].p + 1;
-        const double rs = 4.0 * q * (q + 1) * (2 * q + 1) / 6.0;
-        f[1 + k] += 2.0 * 3.0 * rs * g.npair;
-      } else {
-        double dim = ops_->dims[g.group];
-        f[1 + k] += 2.0 * dim * dim * g.npair;
-      }
-    }
+    for (const TransSeg& g : S[k]->segs) f[1 + k] += pair_flops(g.group, false) * g.npair;
   f[4] = 2.0 * D * 9.0 * (double)(n_ + nt_);  // 9 derivative sums per point
+}
+
+// Flops of one translation of group g for one column in the form that runs.
+double Plan::pair_flops(int g, bool mixed) const {
+  const double q = ops_->descs[g].p + 1, D = 2.0 * ncoef(p_);
+  auto s2 = [](double x) { return x * (x + 1) * (2 * x + 1) / 6.0; };
+  const bool fact = factored_ && (mixed ? 2.0 * D * rot_cols_per_cta((int)D, 4) * 4 <= 227.0 * 1024 : rot_mma_ok(p_));
+  // parity-split form: two Ry of sum_n (n+1)^2 + n^2, the shift's re and im
+  // blocks (none of order 0 im), two Rz of 4 per coefficient of order m > 0 (1
+  // for m = 0) multiply-adds
+  if (fact && (!mixed || (split_rot() && q <= 32)))
+    return 2.0 * (2.0 * (s2(q) + s2(q - 1)) + 2.0 * s2(q) - q * q + 2.0 * (4.0 * (q * (q + 1) / 2 - q) + q));
+  // full blocks: two rotations and the shift, sum_{j=1}^{p+1} (2j)^2 each
+  if (fact) return 2.0 * 3.0 * 4.0 * s2(q);
+  const double dim = ops_->dims[g];
+  return 2.0 * dim * dim;
 }
 
 void Plan::set_mixed_floor(double eps) {
@@ -1492,26 +1496,8 @@ void Plan::translation_flops(int R, bool mixed, double* f) {
   if (!far_) return;
   MixedOrders orders(this, mixed);
   ensure_ops();
-  const double D = 2.0 * ncoef(p_);
-  const bool fact = factored_ && 2.0 * D * rot_cols_per_cta((int)D, 4) * 4 <= 227.0 * 1024;
-  // the parity-split form (FP32): per column two Ry of sum_n (n+1)^2 + n^2,
-  // the shift's re and im blocks (none of order 0 im), two Rz of 4 per
-  // coefficient of order m > 0 (1 for m = 0) multiply-adds
-  const bool split = mixed && split_rot();
-  auto s2 = [](double x) { return x * (x + 1) * (2 * x + 1) / 6.0; };
   auto add = [&](const TransSched& S, int k, double cols) {
-    for (const TransSeg& g : S.segs) {
-      const double q = ops_->descs[g.group].p + 1;
-      if (fact && split && q <= 32) {
-        const double ma = 2.0 * (s2(q) + s2(q - 1)) + 2.0 * s2(q) - q * q + 2.0 * (4.0 * (q * (q + 1) / 2 - q) + q);
-        f[k] += 2.0 * ma * g.npair * cols;
-      } else if (fact) {
-        f[k] += 2.0 * 3.0 * (4.0 * q * (q + 1) * (2 * q + 1) / 6.0) * g.npair * cols;
-      } else {
-        const double dim = ops_->dims[g.group];
-        f[k] += 2.0 * dim * dim * g.npair * cols;
-      }
-    }
+    for (const TransSeg& g : S.segs) f[k] += pair_flops(g.group, mixed) * g.npair * cols;
   };
   if (!mindlin_) {
     add(m2m_, 0, 4.0 * R);

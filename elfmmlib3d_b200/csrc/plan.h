@@ -245,9 +245,8 @@ class Plan {
   void flops_per_column(double* f5) const;
   // Flops of one pass's translation launches for R right-hand sides at the
   // orders of the given form (mixed: the mixed form's orders and pool):
-  // f3 = M2M, M2L, L2L (factored form: two rotations and the z shift per
-  // pair and column; dense: 2 dim^2); image: the image plan's schedules
-  // (6R Laplace columns, R columns of U with its dense M2L).
+  // f3 = M2M, M2L, L2L (pair_flops per pair and column); image: the image
+  // plan's schedules (6R Laplace columns, R columns of U with its own M2L).
   void translation_flops(int R, bool mixed, double* f3);
   // all-pairs direct sum on the same geometry (no tree needed)
   // nsub > 0: only the first nsub source points (centroids), no targets
@@ -286,6 +285,7 @@ class Plan {
     DevBuf<NearTask> t;
     int n = 0, key = -1;
   };
+  double pair_flops(int g, bool mixed) const;
   const NearTasks& near_tasks(int do_src, int do_tgt, int pts, bool far);
   bool mindlin_ = false, img_sched_ = false;
   bool forest_on_ = false;

@@ -413,9 +413,10 @@ int efmm_plan_set_mixed_floor(efmm_plan *plan, double eps, int *order);
 
 /* Flops of one pass's translation launches (M2M, M2L, L2L into f3) for
  * nrhs right-hand sides at the orders of the form `precision` selects
- * (1: the mixed form's), counted as the kernels run them (factored: two
- * rotations and the shift along z per pair and column).  Measurement
- * support, no counterpart in the reference. */
+ * (1: the mixed form's), counted as the kernels run them (per pair and
+ * column the blocks of the parity-split form, of the full-block form or of
+ * the dense operator).  Measurement support, no counterpart in the
+ * reference. */
 int efmm_plan_translation_flops(efmm_plan *plan, int nrhs, int precision, double *f3);
 
 /* Direct sum at the first nsub source points only (centroids 0..nsub-1,
