@@ -363,10 +363,10 @@ def make_uneven_problems(w, world=1, rank=None):
 
 
 # FP64 operations per near-field (point, triangle) pair of the analytic
-# kernel: ncu thread-instruction counts of k_near_leaf on the sphere-5120 case,
-# (dadd + dmul + 2 dfma) / pairs = (0.999e9 + 1.749e9 + 2 * 3.029e9) / 3.193e6
-# (profiles/near_leaf_sphere5120.md)
-NEAR_FLOPS_PER_PAIR = 2758.0
+# kernel, both layers with strain: ncu thread-instruction counts of k_near_leaf
+# on the sphere-5120 case, (dadd + dmul + 2 dfma) / pairs = (0.305e9 + 1.154e9 +
+# 2 * 1.750e9) / 3.193e6 (profiles/near_leaf_sphere5120.md)
+NEAR_FLOPS_PER_PAIR = 1553.0
 
 
 def run_ours(args, rank, world, local_rank):
