@@ -24,11 +24,19 @@
 // Compared with derivative tables of the integrals of r and 1/r in the
 // triangle frame (45 entries per pair, as the reference's triartable and
 // triabtable, src/triahquad.f:680 and :797, rotated per edge, then contracted,
-// the form used before): about half the FP64 operations and two thirds of the
-// registers, errors against long double equal to within 1.3x from 1 to 30
-// edge lengths.  On-surface evaluation (target on its own triangle) uses h =
-// 0, Omega = 0: the principal value / Hadamard finite part, the reference's
-// iquad = 0 convention (src/triahquad.f:4037-4055).
+// the form used before): 1,553 FP64 operations per pair of both layers instead
+// of 2,758 and two thirds of the registers.  Errors against 113 bits (rms over
+// random and thin triangles, heights down to 1e-4 of the base, with fused
+// multiply-adds as on the device) beside those of the tables: off the plane 0.05
+// to 1.3 times theirs, near it the double layer's strain up to 1.5; close to a
+// vertex 1e-2 to 1e-9 of theirs (u and v from the nearer end of an edge), to an
+// edge 0.2 to 1.  In the triangle's plane (every planar fault) the single layer
+// 0.3 to 1.5; the double layer's sums over the edges cancel further out: 0.1 to
+// 1.8 within 3 edge lengths, 0.6 to 2.2 from 10 to 100 (displacement at 30:
+// 1.3e-12 against 0.9e-12).
+// On-surface evaluation (target on its own triangle) uses h = 0, Omega = 0: the
+// principal value / Hadamard finite part, the reference's iquad = 0 convention
+// (src/triahquad.f:4037-4055).
 #pragma once
 #include "tri_index.cuh"
 
@@ -120,18 +128,29 @@ EFMM_HD void te_line(double len, double uA, double uB, double RA, double RB, dou
 // Offsets r from the vertices to X, distances R and their reciprocals, 0 at a
 // vertex itself (the ends' terms that diverge there are left out as the
 // edge's are).  Returns the signed distance from the plane, 0 for the
-// centroid (self) and at a vertex.
+// centroid (self); measured from the nearest vertex it has the rounding of
+// that distance and is 0 at a vertex.
 EFMM_HD double te_vertices(const TriEdge& T, const double* X, bool self, double r[3][3], double R[3], double iR[3]) {
-  bool flat = self;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
 #pragma unroll
     for (int c = 0; c < 3; c++) r[k][c] = X[c] - T.v[3 * k + c];
     R[k] = sqrt(te_dot(r[k], r[k]));
     iR[k] = R[k] > 0.0 ? 1.0 / R[k] : 0.0;
-    flat = flat || R[k] == 0.0;
   }
-  return flat ? 0.0 : te_dot(r[0], T.n);
+  const bool n1 = R[1] < R[0], n2 = R[2] < (n1 ? R[1] : R[0]);
+  double d[3];
+#pragma unroll
+  for (int c = 0; c < 3; c++) d[c] = n2 ? r[2][c] : (n1 ? r[1][c] : r[0][c]);
+  return self ? 0.0 : te_dot(d, T.n);
+}
+
+// Offset from the nearer end of edge k to X (no dynamic register indexing);
+// nb: that is its end B.
+EFMM_HD void te_near_end(int k, bool nb, const double r[3][3], double d[3]) {
+  const bool i0 = nb ? k == 2 : k == 0, i1 = nb ? k == 0 : k == 1;
+#pragma unroll
+  for (int c = 0; c < 3; c++) d[c] = i0 ? r[0][c] : (i1 ? r[1][c] : r[2][c]);
 }
 
 // Response at X of one triangle: displacement u[3] and strain e[6] (if STR),
@@ -156,20 +175,18 @@ EFMM_HD void tri_edge_pair(const TriEdge& T, const double* X, bool self, bool st
   for (int k = 0; k < 3; k++) {
     const double* t = T.t + 3 * k;
     const double len = T.len[k];
-    // both ends of the edge without dynamic register indexing
-    double rA[3], RA, RB, iA, iB;
-#pragma unroll
-    for (int c = 0; c < 3; c++) rA[c] = k == 0 ? r[0][c] : (k == 1 ? r[1][c] : r[2][c]);
-    RA = k == 0 ? R[0] : (k == 1 ? R[1] : R[2]);
-    RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
-    iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
-    iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
-    // (exactly 0 at an end: the products round)
-    const bool end = RB == 0.0;
-    const double uA = end ? len : te_dot(rA, t), uB = end ? 0.0 : uA - len;
-    double nu[3];
+    // both ends of the edge; u and v from the nearer one, with its rounding (at
+    // an end itself both are exactly 0)
+    const double RA = k == 0 ? R[0] : (k == 1 ? R[1] : R[2]);
+    const double RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
+    const double iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
+    const double iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
+    const bool nb = RB < RA;
+    double d[3], nu[3];
+    te_near_end(k, nb, r, d);
+    const double ud = te_dot(d, t), uA = nb ? ud + len : ud, uB = nb ? ud : ud - len;
     te_cross(t, T.n, nu);
-    const double v = end ? 0.0 : te_dot(rA, nu);
+    const double v = te_dot(d, nu);
     const double rho[3] = {v * nu[0] + h * T.n[0], v * nu[1] + h * T.n[1], v * nu[2] + h * T.n[2]};
     const double c2 = v * v + h * h;
     double L, K3, K5;
@@ -260,21 +277,20 @@ struct TeEdge {
 };
 EFMM_HD void te_edge(const TriEdge& T, int k, const double r[3][3], const double R[3], const double iR[3], double h,
                      TeEdge& g) {
-  double rA[3];
 #pragma unroll
-  for (int c = 0; c < 3; c++) {
-    rA[c] = k == 0 ? r[0][c] : (k == 1 ? r[1][c] : r[2][c]);
-    g.t[c] = T.t[3 * k + c];
-  }
+  for (int c = 0; c < 3; c++) g.t[c] = T.t[3 * k + c];
   g.RA = k == 0 ? R[0] : (k == 1 ? R[1] : R[2]);
   g.RB = k == 0 ? R[1] : (k == 1 ? R[2] : R[0]);
   g.iA = k == 0 ? iR[0] : (k == 1 ? iR[1] : iR[2]);
   g.iB = k == 0 ? iR[1] : (k == 1 ? iR[2] : iR[0]);
-  const bool end = g.RB == 0.0;
-  g.uA = end ? T.len[k] : te_dot(rA, g.t);
-  g.uB = end ? 0.0 : g.uA - T.len[k];
+  const bool nb = g.RB < g.RA;
+  double d[3];
+  te_near_end(k, nb, r, d);
+  const double ud = te_dot(d, g.t);
+  g.uA = nb ? ud + T.len[k] : ud;
+  g.uB = nb ? ud : ud - T.len[k];
   te_cross(g.t, T.n, g.nu);
-  g.v = end ? 0.0 : te_dot(rA, g.nu);
+  g.v = te_dot(d, g.nu);
   g.h = h;
 #pragma unroll
   for (int c = 0; c < 3; c++) g.rho[c] = g.v * g.nu[c] + h * T.n[c];

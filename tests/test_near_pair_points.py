@@ -113,3 +113,32 @@ def test_device_on_edges(gpu):
         assert np.isfinite(got).all()
         if layer == 0:
             assert rel(got[:, :3], ref[:, :3]) < 1e-12
+
+
+@pytest.mark.parametrize("dist", [1e-2, 1e-4, 1e-6])
+@pytest.mark.parametrize("height", [0.7, 0.02])
+def test_close_to_a_corner_in_the_plane(lib, dist, height):
+    """The pair does not depend on the order of the vertices (an odd one turns
+    the normal, and the double layer's sign).  Close to a corner
+    in the triangle's plane that holds only if the point's distances from the
+    edges are measured from the nearer end: from the far one their rounding is
+    that of the edge's length, 1e-16 / dist of the result and, in the strain of
+    the double layer, its square root's worth more.  Some dozens of roundings
+    of terms up to 1 / height times their sum: 1e-12."""
+    rng = np.random.default_rng(7)
+    worst = 0.0
+    for _ in range(60):
+        a = rng.normal(size=2)
+        t = rng.uniform(0, 2 * np.pi)
+        e, n = np.array([np.cos(t), np.sin(t)]), np.array([-np.sin(t), np.cos(t)])
+        tri = np.zeros((3, 3))
+        tri[:, :2] = a, a + e, a + rng.uniform(0.2, 0.8) * e + height * n
+        phi = rng.uniform(0, 2 * np.pi)
+        x = tri[rng.integers(3)] + dist * np.array([np.cos(phi), np.sin(phi), 0.0])
+        s = rng.normal(size=3)
+        for ab in ((s, None), (None, s)):
+            f = 1.0 if ab[1] is None else -1.0
+            o = _pair(lib, tri, *ab, x)
+            for order in ((0, 2, 1), (1, 0, 2), (2, 1, 0)):
+                worst = max(worst, *(rel(v, f * w) for v, w in zip(o, _pair(lib, tri[list(order)], *ab, x))))
+    assert worst < 1e-12
