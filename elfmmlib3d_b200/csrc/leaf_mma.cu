@@ -347,13 +347,13 @@ template <class T, bool IMG>
 bool launch_p2m_mma(cudaStream_t st, int nleaf, const P2MArgs& a, int R, long long ubase, T* mpole) {
   // 8 warps of 12 row tiles, two CTAs per SM, to order 26; 16 warps of 8 row
   // tiles to order 30; above, 16 warps of 14 row tiles and 8 columns at a
-  // time (FP64 only: a column's weights fall in two groups, which add up)
+  // time (FP64 only: a column's weights fall in two groups, which add up) to
+  // order 39, the last whose harmonics fit in shared memory
   const int p = a.p;
-  if (p > 40 || (p > 30 && sizeof(T) == 4)) return false;
+  if (p > 39 || (p > 30 && sizeof(T) == 4)) return false;
   if (nleaf <= 0 || R <= 0) return true;
   const int nt = p > 30 ? 1 : 2, ng = p2m_groups(nt, IMG);
   const size_t smem = p2m_mma_smem(p, nt);
-  if (smem > 227 * 1024) return false;
   // parts of the nodes while leaves x groups leave the chip (two CTAs per SM,
   // four rounds) unfilled; each part pays the table and the final shifts
   int parts = 1;

@@ -20,7 +20,7 @@
 // all its inputs are read, and takes the operator from L2 in fragment order
 // (256 contiguous bytes per 8 x 4 tile, zero padded, one k step ahead).
 //
-// Columns per CTA: 32 while the rows fit (p <= 28), else 16; fewer where a
+// Columns per CTA: 32 while the rows fit (p <= 29), else 16; fewer where a
 // launch's groups are so small that most of a tile would be padding.
 //
 // What bounds it is the FP64 tensor pipe and, between its bursts, the latency
