@@ -48,12 +48,14 @@ __global__ void k_tri_edge_prep(int n, const double* __restrict__ tri, const dou
 // warp and lanes over the triangles of one box at a time, on derivative
 // tables (228 registers, half of the lanes idle), took 104 ms on 327,680
 // triangles + 250,007 targets at iprec 2 (165 M pairs) and 2.66 ms on 317 + 41
-// (about 20 leaves); this form 18.3 ms and 0.058 ms.  Items instead of
+// (about 20 leaves); this form 19.1 ms and 0.058 ms.  Items instead of
 // whole leaves matter where a few leaves hold most pairs (a coarse target
 // leaf beside hundreds of fine source boxes): whole leaves took 12.5 ms
 // against 6.0 on 81,920 triangles + 62,501 shell targets (55 M pairs).
-// Registers for 3 CTAs per SM: 2, 4 and 5 measured 23.6, 18.6 and 19.8 ms on
-// the large case, 1.23, 1.31 and 1.54 ms against 1.15 on 5,120 + 1,000.
+// Registers for 3 CTAs per SM: 2, 3, 4 and 5 measured 23.6, 18.3, 18.6 and 19.8
+// ms on the large case, 1.23, 1.15, 1.31 and 1.54 ms on 5,120 + 1,000 (before
+// items, and before points at vertices, on edges and near corners were told
+// apart).
 // Outputs are ADDED to u (3/pt) and e (6/pt, xx yy zz xy xz yz).
 constexpr int NL_THREADS = NEAR_TASK_PTS, NL_TILE = 32, NL_STRIDE = 34;  // record stride (doubles) free of bank conflicts
 
@@ -526,7 +528,7 @@ k_near_batch(const NearArgs a, const NearTask* __restrict__ tasks, int R, int K,
 // inner loop unrolled.  Same tiling as k_near_batch (work items of 8 points, 16
 // triangles per tile, 9 x RB outputs per thread).  Items instead of whole
 // lists: the image replay of 64 right-hand sides on 18,034 triangles, where few
-// points have near triangles, 10.5 -> 4.1 ms.  The next tile's triangles are
+// points have near triangles, 10.5 -> 2.8 ms.  The next tile's triangles are
 // looked up while this one's are read, so that a tile costs two barriers, and
 // the densities are read before the store: 5 right-hand sides, near field alone
 // of 5,120 triangles + 1,000 targets 12.5 ms (three barriers 21, the store
@@ -984,7 +986,7 @@ void launch_near_batch(cudaStream_t st, const NearArgs& a, int ntask, const Near
 
 // Up to this many right-hand sides the store is streamed (k_near_replay):
 // 18,034 triangles, iprec 3 (about 16 GB): 3.4 ms for 2 and 6.3 for 4 against
-// 14.0 ms of k_near_replay_batch for any number up to 16.
+// 8.7 ms of k_near_replay_batch for any number up to 16.
 constexpr int NEAR_STREAM_R = 4;
 void launch_near_replay_batch(cudaStream_t st, const NearArgs& a, int ntask, const NearTask* tasks, int R,
                               int dostrain, const double* ssl, const double* sdl, int nsrc, int ntgt,

@@ -51,7 +51,7 @@ double iprec_eps(int iprec) {
 // Up to this many right-hand sides the analytic near field runs once per
 // right-hand side (densities contracted per pair) instead of once for all
 // (unit responses, then the product): 0.75 ms each against 4.0 ms on 9,973
-// triangles + 2,003 targets, 0.052 against 0.232 on 1,000 triangles, 6.0
+// triangles + 2,003 targets, 0.052 against 0.232 on 1,000 triangles, 6.3
 // against 30.8 on 81,920 + 62,501, iprec 2, both layers with strain.
 constexpr int NEAR_LEAF_R = 4;
 
